@@ -2040,7 +2040,6 @@ static std::vector<bs_volume*> batch_core(bs_ctx* ctx, const float* d_xyz, const
   DBuf<uint32_t> act(ctx, std::max<uint64_t>(na, 1));
   if (nb) BS_KERNEL(ctx, "k_emit_active", (k_emit_active<<<blocks(nb * 32, 256), 256, 0, s>>>(masks.p, voff.p, nb, act.p)));
   vc.reset();
-  voff.reset();
 
   // join the tree build; the triangles are freed after it
   BS_CUDA(cudaStreamWaitEvent(s, built.e, 0));
@@ -2053,7 +2052,7 @@ static std::vector<bs_volume*> batch_core(bs_ctx* ctx, const float* d_xyz, const
     DBuf<unsigned long long> d_cnt(ctx, 6);
     BS_CUDA(cudaMemcpyAsync(d_rm.p, rm.data(), K * sizeof(RefSignMesh), cudaMemcpyHostToDevice, s));
     BS_CUDA(cudaMemsetAsync(d_cnt.p, 0, 6 * sizeof(unsigned long long), s));
-    ref_tree_sign(ctx, rt, act.p, act_base.p, d_wb.p, warp_base[K], K, d_rm.p, origins.p, values.p, d_cnt.p);
+    ref_tree_sign(ctx, rt, act.p, voff.p, nb, na, act_base.p, leaf_base.p, K, d_rm.p, origins.p, values.p, d_cnt.p);
     read_back(ctx, rt_cnt, d_cnt.p, sizeof rt_cnt);
     if (rt_cnt[3]) fail(BS_ERR_CAPACITY, "winding-number traversal stack overflow");
   } else if (na > 0) {

@@ -42,6 +42,7 @@
 #include <vector>
 
 #include "ref_tree.cuh"
+#include "solid_angle.cuh"
 
 namespace bs {
 namespace {
@@ -912,33 +913,6 @@ __global__ void k_rt_open(uint64_t nt, const int* __restrict__ flags, const int2
 }
 
 // ------------------------------------------------------------ traversal ---
-// v / len for the three components of v, correctly rounded, with one
-// reciprocal (mdiv) where the operands allow it.
-__device__ __forceinline__ F3 div3(F3 v, float len) {
-  if (mdiv_range(len) && (v.x == 0.0f || mdiv_range(v.x)) && (v.y == 0.0f || mdiv_range(v.y)) &&
-      (v.z == 0.0f || mdiv_range(v.z))) {
-    const float y = __frcp_rn(len);
-    // a zero component keeps its sign (0 / len = 0 * (1 / len))
-    return f3(v.x == 0.0f ? fmul(v.x, y) : mdiv(v.x, len, y), v.y == 0.0f ? fmul(v.y, y) : mdiv(v.y, len, y),
-              v.z == 0.0f ? fmul(v.z, y) : mdiv(v.z, len, y));
-  }
-  return f3(fdiv(v.x, len), fdiv(v.y, len), fdiv(v.z, len));
-}
-
-// solid_angle (aabb_tree.rs:582-615): Van Oosterom–Strackee, unfused.
-__device__ __forceinline__ float solid_angle(float4 A, float4 Bv, float4 C, F3 q) {
-  F3 qa = sub3(f3(A.x, A.y, A.z), q), qb = sub3(f3(Bv.x, Bv.y, Bv.z), q), qc = sub3(f3(C.x, C.y, C.z), q);
-  const float la = fsqrt(dot3(qa, qa)), lb = fsqrt(dot3(qb, qb)), lc = fsqrt(dot3(qc, qc));
-  if (la == 0.f || lb == 0.f || lc == 0.f) return 0.f;
-  qa = div3(qa, la);
-  qb = div3(qb, lb);
-  qc = div3(qc, lc);
-  const float num = dot3(qa, cross3(sub3(qb, qa), sub3(qc, qa)));
-  if (num == 0.f) return 0.f;
-  const float den = fadd(fadd(fadd(1.0f, dot3(qa, qb)), dot3(qa, qc)), dot3(qb, qc));
-  return fmul(atan2f(num, den), 2.0f);
-}
-
 // Far field of a node at q (aabb_tree.rs:666-671 with hessians, 803-816):
 // r = p - q, the order-1 term a . r / (4 pi |r|^3) and the Frobenius product
 // of the order-2 coefficients with I / (4 pi |r|^3) - 3 r r^T / (4 pi |r|^5).
@@ -1132,45 +1106,46 @@ __device__ __forceinline__ void flush_counts(const Counts& c, unsigned long long
   }
 }
 
-constexpr int SIGN_WARPS = 4;
+constexpr int SIGN_WARPS = REF_SIGN_WARPS;
 
-// One warp per 32 consecutive band voxels of one mesh (mesh_to_volume.rs:
-// 245-280): warps are numbered per mesh (warp_base[m] .. warp_base[m+1]).
-// WARPS per block: 2, 4 or 8 (the context's tuned launch shape).
-template <int WARPS>
-__global__ void __launch_bounds__(32 * WARPS) k_rt_sign(const uint32_t* __restrict__ act,
-                                                             const uint32_t* __restrict__ act_base,
-                                                             const uint32_t* __restrict__ warp_base, int K,
-                                                             const RefSignMesh* __restrict__ meshes,
-                                                             const int4* __restrict__ origins,
-                                                             float* __restrict__ values,
-                                                             const float4* __restrict__ rec_i,
-                                                             const float4* __restrict__ opn,
-                                                             const float4* __restrict__ rec_l,
-                                                             const uint32_t* __restrict__ leaf_cnt,
-                                                             const float4* __restrict__ tri,
-                                                             unsigned long long* __restrict__ counters) {
-  __shared__ WarpStack ws[WARPS];
+// The band voxels the filter left undecided (mesh_to_volume.rs:245-280): a
+// warp takes a few of one mesh at a time; the lists' lengths are on the
+// device, so a grid of resident blocks walks them.
+__global__ void __launch_bounds__(32 * SIGN_WARPS) k_rt_sign_exact(const uint32_t* __restrict__ list,
+                                                                   const uint32_t* __restrict__ list_base,
+                                                                   const uint32_t* __restrict__ count,
+                                                                   const uint32_t* __restrict__ warp_base, int K,
+                                                                   const RefSignMesh* __restrict__ meshes,
+                                                                   const int4* __restrict__ origins,
+                                                                   float* __restrict__ values,
+                                                                   const float4* __restrict__ rec_i,
+                                                                   const float4* __restrict__ opn,
+                                                                   const float4* __restrict__ rec_l,
+                                                                   const uint32_t* __restrict__ leaf_cnt,
+                                                                   const float4* __restrict__ tri,
+                                                                   unsigned long long* __restrict__ counters) {
+  __shared__ WarpStack ws[SIGN_WARPS];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const uint64_t gw = blockIdx.x * uint64_t(WARPS) + w;
-  if (gw >= warp_base[K]) return;  // whole warp
-  const int m = K > 1 ? mesh_of(warp_base, K, gw) : 0;
-  const uint64_t a1 = act_base[m + 1];
-  const uint64_t i = act_base[m] + (gw - warp_base[m]) * 32 + lane;
-  const bool ok = i < a1;
-  const RefSignMesh M = meshes[m];
-  const uint32_t v = act[ok ? i : a1 - 1];
-  const uint32_t b = v >> 9, o = v & 511;
-  const int4 org = origins[b];
-  const F3 q = f3(fmul(__int2float_rn(org.x + int(o >> 6)), M.h), fmul(__int2float_rn(org.y + int((o >> 3) & 7)), M.h),
-                  fmul(__int2float_rn(org.z + int(o & 7)), M.h));
-  Counts c;
-  const float wn = ref_wn_warp(q, __ballot_sync(FULL, ok), M.root, rec_i, opn, rec_l, leaf_cnt, tri, ws[w], c);
-  if (ok) {
-    const float d = values[uint64_t(b) * 512 + o];
-    values[uint64_t(b) * 512 + o] = (wn < M.thresh) ? copysignf(d, 1.0f) : copysignf(d, -1.0f);
+  const uint32_t n_warps = warp_base[K], per = warp_base[K + 1];
+  for (uint64_t gw = blockIdx.x * uint64_t(SIGN_WARPS) + w; gw < n_warps; gw += uint64_t(gridDim.x) * SIGN_WARPS) {
+    const int m = K > 1 ? mesh_of(warp_base, K, gw) : 0;
+    const uint32_t i = uint32_t(gw - warp_base[m]) * per + lane, n = count[m];
+    const bool ok = uint32_t(lane) < per && i < n;
+    const RefSignMesh M = meshes[m];
+    const uint32_t v = list[uint64_t(list_base[m]) + (ok ? i : n - 1)];
+    const uint32_t b = v >> 9, o = v & 511;
+    const int4 org = origins[b];
+    const F3 q = f3(fmul(__int2float_rn(org.x + int(o >> 6)), M.h), fmul(__int2float_rn(org.y + int((o >> 3) & 7)), M.h),
+                    fmul(__int2float_rn(org.z + int(o & 7)), M.h));
+    Counts c;
+    const float wn = ref_wn_warp(q, __ballot_sync(FULL, ok), M.root, rec_i, opn, rec_l, leaf_cnt, tri, ws[w], c);
+    if (ok) {
+      const float d = values[uint64_t(b) * 512 + o];
+      values[uint64_t(b) * 512 + o] = (wn < M.thresh) ? copysignf(d, 1.0f) : copysignf(d, -1.0f);
+    }
+    if (lane == 0 && c.overflow) atomicAdd(counters + 3, 1ull);
+    __syncwarp();
   }
-  flush_counts(c, counters);
 }
 
 __global__ void __launch_bounds__(32 * SIGN_WARPS) k_rt_points(const float* __restrict__ pts, uint64_t np, int root,
@@ -1321,21 +1296,19 @@ void ref_tree_set_beta(bs_ctx* ctx, RefTrees& t, const std::vector<float>& beta)
   t.h_beta = beta;
 }
 
-void ref_tree_sign(bs_ctx* ctx, const RefTrees& t, const uint32_t* act, const uint32_t* d_act_base,
-                   const uint32_t* d_warp_base, uint64_t n_warps, int K, const RefSignMesh* d_meshes,
-                   const int4* origins, float* values, unsigned long long* d_counters) {
-  if (n_warps == 0) return;
-#define BS_RT_SIGN(W)                                                                                        \
-  BS_KERNEL(ctx, "k_rt_sign", (k_rt_sign<W><<<nblk(n_warps, W), 32 * W, 0, ctx->stream>>>(                   \
-                                  act, d_act_base, d_warp_base, K, d_meshes, origins, values, t.rec_i.p, t.open.p, \
-                                  t.rec_l.p, t.leaf_cnt.p, t.tri.p, d_counters)))
-  if (ctx->tune_wn_warps == 2)
-    BS_RT_SIGN(2);
-  else if (ctx->tune_wn_warps == 8)
-    BS_RT_SIGN(8);
-  else
-    BS_RT_SIGN(4);
-#undef BS_RT_SIGN
+unsigned ref_tree_sign_exact_grid(bs_ctx* ctx, uint64_t max_list) {
+  int n_sm = 0;
+  BS_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, ctx->device));
+  return unsigned(std::min<uint64_t>(nblk(max_list, SIGN_WARPS), uint64_t(n_sm) * 8));
+}
+
+void ref_tree_sign_exact(bs_ctx* ctx, const RefTrees& t, unsigned grid, const uint32_t* list,
+                         const uint32_t* d_list_base, const uint32_t* d_count, const uint32_t* d_warps, int K,
+                         const RefSignMesh* d_meshes, const int4* origins, float* values,
+                         unsigned long long* d_counters) {
+  BS_KERNEL(ctx, "k_rt_sign_exact", (k_rt_sign_exact<<<grid, 32 * SIGN_WARPS, 0, ctx->stream>>>(
+                                        list, d_list_base, d_count, d_warps, K, d_meshes, origins, values, t.rec_i.p,
+                                        t.open.p, t.rec_l.p, t.leaf_cnt.p, t.tri.p, d_counters)));
 }
 
 void ref_tree_points(bs_ctx* ctx, RefTrees& t, const float* d_pts, uint64_t np, float beta, float* d_out,

@@ -49,17 +49,29 @@ struct RefSignMesh {
   float h, beta, thresh;
 };
 
-// Signs the active voxels of K meshes (act[i] = brick << 9 | voxel; mesh m
-// owns act[act_base[m], act_base[m+1]) and warps warp_base[m] ..
-// warp_base[m+1] of 32 voxels each) with the winding number of their grid
-// points: values[v] = +|d| when wn < thresh, else -|d|
-// (mesh_to_volume.rs:245-280).  counters (device, 6 x u64, accumulated):
-// warp node visits, far-field evaluations, exact solid angles, stack
-// overflows, far-field evaluations and exact solid angles as the warps run
-// them (a section any lane needs runs for the whole warp).
-void ref_tree_sign(bs_ctx* ctx, const RefTrees& t, const uint32_t* act, const uint32_t* d_act_base,
-                   const uint32_t* d_warp_base, uint64_t n_warps, int K, const RefSignMesh* d_meshes,
-                   const int4* origins, float* values, unsigned long long* d_counters);
+// Signs the active voxels of K meshes (act[i] = brick << 9 | voxel, brick b
+// owning act[voff[b], voff[b+1]) in Morton order; mesh m owns bricks
+// [leaf_base[m], leaf_base[m+1]) and act[act_base[m], act_base[m+1])) with the
+// winding number of their grid points: values[v] = +|d| when wn < thresh,
+// else -|d| (mesh_to_volume.rs:245-280).  sign_filter.cu settles all but a few
+// voxels; the rest take the exact traversal.  counters (device, 6 x u64,
+// accumulated): node visits, far-field evaluations and exact solid angles of
+// the voxels' own cuts, stack overflows, far-field evaluations and solid
+// angles as the kernel runs them (one for a whole group of voxels).
+void ref_tree_sign(bs_ctx* ctx, const RefTrees& t, const uint32_t* act, const uint32_t* voff, uint64_t n_bricks,
+                   uint64_t n_act, const uint32_t* d_act_base, const uint32_t* d_leaf_base, int K,
+                   const RefSignMesh* d_meshes, const int4* origins, float* values, unsigned long long* d_counters);
+
+// The exact traversal for the listed voxels: mesh m's are d_count[m] from
+// list[d_list_base[m]], in warps d_warps[m] .. d_warps[m+1] of d_warps[K + 1]
+// voxels each (device arrays).  Only counters[3] is touched.  grid: resident
+// blocks of REF_SIGN_WARPS warps for at most max_list voxels.
+constexpr int REF_SIGN_WARPS = 4;
+unsigned ref_tree_sign_exact_grid(bs_ctx* ctx, uint64_t max_list);
+void ref_tree_sign_exact(bs_ctx* ctx, const RefTrees& t, unsigned grid, const uint32_t* list,
+                         const uint32_t* d_list_base, const uint32_t* d_count, const uint32_t* d_warps, int K,
+                         const RefSignMesh* d_meshes, const int4* origins, float* values,
+                         unsigned long long* d_counters);
 
 // WindingNumbers::approximate (aabb_tree.rs:654-660) at np device points of
 // mesh 0's tree.

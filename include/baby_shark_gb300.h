@@ -92,8 +92,8 @@ bs_status bs_ctx_last_stats(const bs_ctx* ctx, uint64_t* out8);
  * solid angles of the winding-number pass in 64 bits (per voxel or point on
  * the reference's tree, per warp on the library's PLOC tree), [12] which tree
  * (0 the reference's, 1 PLOC), [13] and [14] on the reference's tree the
- * far-field evaluations and solid angles as its warps execute them (a
- * section that any lane of a warp needs runs for all 32), [15] zero. */
+ * far-field evaluations and solid angles as the pass runs them (once for a
+ * whole group of voxels that share them), [15] zero. */
 enum bs_stats_kind {
   BS_STATS_NONE = 0,
   BS_STATS_MESH_TO_VOLUME = 1,
