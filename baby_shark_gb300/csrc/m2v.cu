@@ -1632,7 +1632,15 @@ struct SideStream {
   bs_ctx* ctx;
   cudaStream_t main;
   explicit SideStream(bs_ctx* c) : ctx(c), main(c->stream) {
-    if (!ctx->side) BS_CUDA(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
+    if (!ctx->side) {
+      // above the main stream: the build is a chain of short dependent kernels
+      // beside one long one whose blocks fill the GPU; at equal priority every
+      // build kernel waits for that kernel's last block, above it a build
+      // kernel takes the next free block slots
+      int least = 0, greatest = 0;
+      BS_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+      BS_CUDA(cudaStreamCreateWithPriority(&ctx->side, cudaStreamNonBlocking, greatest));
+    }
     ctx->stream = ctx->side;
   }
   ~SideStream() {
