@@ -193,17 +193,18 @@ extern "C" bs_status bs_dual_contour_noalloc(int device, void* stream, const int
     int* hvals = c.take<int>(DCNA_HASH_CAP);
     int* herr = c.take<int>(1);
     DcStats* st = c.take<DcStats>(1);
-    uint32_t* cm = c.take<uint32_t>(n * 3 * 16);
+    int* nbr = c.take<int>(n * 27);
+    uint32_t* sgn = c.take<uint32_t>(n * 16);
+    uint2* em = c.take<uint2>(n * 3 * 16);
     uint32_t* ccnt = c.take<uint32_t>(n * 3 + 1);
     uint32_t* coff = c.take<uint32_t>(n * 3 + 1);
     float* pts = c.take<float>(DCNA_MAX_CROSSINGS * 6);
-    uint32_t* cellm = c.take<uint32_t>(n * 16);
+    uint2* cellm = c.take<uint2>(n * 16);
     uint32_t* cellc = c.take<uint32_t>(n + 1);
     uint32_t* celloff = c.take<uint32_t>(n + 1);
     float* cells = c.take<float>(DCNA_MAX_CELLS * 3);
     uint64_t* vcnt = c.take<uint64_t>(n + 1);
     uint64_t* voff = c.take<uint64_t>(n + 1);
-    uint16_t* packed = c.take<uint16_t>(n * 128);
     const size_t temp_bytes = 1u << 20;
     void* temp = c.take<unsigned char>(temp_bytes);
     TileLookup tiles{};
@@ -254,22 +255,22 @@ extern "C" bs_status bs_dual_contour_noalloc(int device, void* stream, const int
     hash.mask = DCNA_HASH_CAP - 1;
     k_hash_insert<<<nblocks(n, 256), 256, 0, s>>>(hash, org, n, herr);
     BS_CUDA(cudaGetLastError());
-    DcVol V{org, d_values, d_masks, hash, tiles};
-    launch_dc_edge_mask(has_tiles, V, n, cm, ccnt, s);
+    DcVol V{org, d_values, d_masks, sgn, nbr, hash, tiles};
+    launch_dc_prepare(V, n, nbr, sgn, s);
+    BS_CUDA(cudaGetLastError());
+    launch_dc_masks(has_tiles, V, n, em, ccnt, cellm, cellc, s);
     BS_CUDA(cudaGetLastError());
     scan_in(s, temp, temp_bytes, ccnt, coff, n * 3 + 1);
     const uint32_t ne = read1(s, coff + n * 3);
     if (ne > DCNA_MAX_CROSSINGS) return BS_ERR_CAPACITY;
-    launch_dc_edge_points(has_tiles, V, n, cm, coff, pts, st, s);
-    BS_CUDA(cudaGetLastError());
-    launch_dc_cell_mask(has_tiles, V, n, cellm, cellc, s);
-    BS_CUDA(cudaGetLastError());
     scan_in(s, temp, temp_bytes, cellc, celloff, n + 1);
     const uint32_t nc = read1(s, celloff + n);
     if (nc > DCNA_MAX_CELLS) return BS_ERR_CAPACITY;
-    k_dc_cell_points<<<unsigned(n), 128, 0, s>>>(V, n, cm, coff, pts, cellm, celloff, cells);
+    launch_dc_edge_points(has_tiles, V, n, em, coff, pts, st, s);
     BS_CUDA(cudaGetLastError());
-    k_dc_quads<<<unsigned(n), 128, 0, s>>>(V, n, cm, cellm, celloff, cells, voxel_size, vcnt, nullptr, packed, nullptr);
+    launch_dc_cell_points(0, V, n, em, coff, pts, cellm, celloff, cells, s);
+    BS_CUDA(cudaGetLastError());
+    launch_dc_quads(V, n, em, coff, cellm, celloff, cells, voxel_size, vcnt, nullptr, nullptr, s);
     BS_CUDA(cudaGetLastError());
     scan_in(s, temp, temp_bytes, vcnt, voff, n + 1);
     const uint64_t nt = read1(s, voff + n);
@@ -278,7 +279,7 @@ extern "C" bs_status bs_dual_contour_noalloc(int device, void* stream, const int
     *n_tris = nt;
     if (nt > capacity) return BS_ERR_CAPACITY;  // *n_tris tells the caller the size to provide
     if (nt) {
-      k_dc_quads<<<unsigned(n), 128, 0, s>>>(V, n, cm, cellm, celloff, cells, voxel_size, nullptr, voff, packed, d_tris);
+      launch_dc_quads(V, n, em, coff, cellm, celloff, cells, voxel_size, nullptr, voff, d_tris, s);
       BS_CUDA(cudaGetLastError());
     }
     BS_CUDA(cudaStreamSynchronize(s));
