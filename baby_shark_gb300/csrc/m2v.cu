@@ -65,6 +65,7 @@ struct M2VStats {
   unsigned long long wn_far;         // warp-level far-field evaluations (internal + leaf dipoles)
   unsigned long long wn_exact;       // warp-level exact solid angles
   unsigned long long n_eval;         // (voxel, sub-triangle) pairs left after culling
+  unsigned long long area16;         // surface in sixteenths of a squared voxel (for choosing the distance pass)
 };
 
 // Per-mesh parameters of a batch.  Triangles of mesh m are [tri_base,
@@ -90,8 +91,8 @@ __device__ __forceinline__ int find_seg(const T* __restrict__ base, int k, uint6
 }
 
 // Adds v to *dst once per warp when every active lane targets the same mesh.
-__device__ __forceinline__ void warp_add(unsigned long long* dst, unsigned long long v, int m) {
-  const unsigned mask = __activemask();
+__device__ __forceinline__ void warp_add(unsigned long long* dst, unsigned long long v, int m,
+                                         unsigned mask = __activemask()) {
   const int leader = __ffs(mask) - 1;
   const int m0 = __shfl_sync(mask, m, leader);
   if (__all_sync(mask, m == m0)) {
@@ -129,18 +130,65 @@ __device__ __forceinline__ void warp_max(T* dst, T v, bool uniform, unsigned mas
 struct SubTri {  // 64 B: vertices, cull coefficients and the widened inclusive integer box
   float4 p0;     // a.x a.y a.z b.x
   float4 p1;     // b.y b.z c.x c.y
-  float4 p2;     // c.z, cull coefficients c2 and E0 (cull_coeffs), -
+  float4 p2;     // c.z, cull coefficients c2, E0 and E1 (cull_coeffs)
   int4 lo;       // box min (x, y, z), mesh
   int4 hi;       // box max
 };
 
+// A triangle's n^2 sub-triangles come in patches of neighbouring ones: the
+// whole triangle for n <= 3, else blocks of 2 x 2 cells (row r, column k <= r,
+// each cell an upright and, for k < r, an inverted sub-triangle).
+__host__ __device__ __forceinline__ uint32_t patch_count(uint32_t n) {
+  const uint32_t m = (n + 1) / 2;
+  return n <= 3 ? 1u : m * (m + 1) / 2;
+}
+
+// Position within its triangle of the sub-triangle in row r, column k.
+__device__ __forceinline__ uint32_t sub_index(uint32_t r, uint32_t k, bool down) {
+  return r * r + (down ? 2 * k : (k == 0 ? 2 * r : 2 * k - 1));
+}
+
+// r with r^2 <= m < (r + 1)^2.
+__device__ __forceinline__ uint32_t isqrt(uint32_t m) {
+  uint32_t r = uint32_t(sqrtf(float(m)));
+  while (uint64_t(r) * r > m) --r;
+  while (uint64_t(r + 1) * (r + 1) <= m) ++r;
+  return r;
+}
+
+// Largest t in [0, n) with off[t] <= i for every thread's own i of a block
+// covering [first, first + blockDim.x): the block's range is searched once,
+// the threads search inside it.
+__device__ __forceinline__ uint64_t owner_of(const uint32_t* __restrict__ off, uint64_t n, uint64_t first, uint64_t i) {
+  __shared__ uint64_t range[2];
+  if (threadIdx.x < 2) {
+    const uint64_t want = threadIdx.x ? first + blockDim.x - 1 : first;
+    uint64_t lo = 0, hi = n - 1;
+    while (lo < hi) {
+      const uint64_t mid = (lo + hi + 1) >> 1;
+      if (uint64_t(__ldg(off + mid)) <= want) lo = mid;
+      else hi = mid - 1;
+    }
+    range[threadIdx.x] = lo;
+  }
+  __syncthreads();
+  uint64_t lo = range[0], hi = range[1];
+  while (lo < hi) {
+    const uint64_t mid = (lo + hi + 1) >> 1;
+    if (uint64_t(__ldg(off + mid)) <= i) lo = mid;
+    else hi = mid - 1;
+  }
+  return lo;
+}
+
 // ------------------------------------------- 1. triangles and subdivision --
 __global__ void k_gather(const float* __restrict__ xyz, const uint32_t* __restrict__ tri, uint64_t nt,
                          const MeshInfo* __restrict__ mi, const uint32_t* __restrict__ tri_base, int K,
-                         float4* __restrict__ T, uint32_t* __restrict__ nsub, M2VStats* st) {
+                         float4* __restrict__ T, uint32_t* __restrict__ nsub, uint32_t* __restrict__ npatch,
+                         M2VStats* st) {
   uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
   if (i >= nt) {
-    if (i == nt) nsub[nt] = 0;
+    if (i == nt) nsub[nt] = npatch[nt] = 0;
     return;
   }
   const int mesh = find_seg(tri_base, K, i);
@@ -151,7 +199,7 @@ __global__ void k_gather(const float* __restrict__ xyz, const uint32_t* __restri
   uint32_t ia = tri[3 * i], ib = tri[3 * i + 1], ic = tri[3 * i + 2];
   if (ia >= M.n_vtx || ib >= M.n_vtx || ic >= M.n_vtx) {
     atomicExch(&S->error, 1);
-    nsub[i] = 0;
+    nsub[i] = npatch[i] = 0;
     T[3 * i] = T[3 * i + 1] = T[3 * i + 2] = make_float4(0, 0, 0, 0);
     return;
   }
@@ -167,18 +215,25 @@ __global__ void k_gather(const float* __restrict__ xyz, const uint32_t* __restri
   float m = fmaxf(fmaxf(dot3(e0, e0), dot3(e1, e1)), dot3(e2, e2));
   float ns = floorf(fdiv(fsqrt(m), h));
   // n^2 sub-triangles in exact integer arithmetic (k_subdivide writes exactly n^2)
-  uint32_t cnt;
+  uint32_t cnt, pc = 1;
   if (!(ns >= 2.0f)) {
     cnt = 1;
   } else if (!(ns < 65536.0f)) {
-    cnt = 0;
+    cnt = pc = 0;
     atomicExch(&S->error, 4);
   } else {
     uint32_t n = uint32_t(ns);
     cnt = n * n;
+    pc = patch_count(n);
   }
   nsub[i] = cnt;
+  npatch[i] = pc;
   warp_add(&S->n_sub, cnt, mesh);
+  {
+    const F3 n = cross3(e0, e1);
+    const float a16 = 8.0f * sqrtf(dot3(n, n)) * inv_h * inv_h;
+    warp_add(&S->area16, a16 < 1e9f ? uint32_t(a16) : 0u, mesh);  // 0 for NaN too
+  }
   F3 mn = min3(c, min3(a, b)), mx = max3(c, max3(a, b));
   float lo[3] = {mn.x, mn.y, mn.z}, hi[3] = {mx.x, mx.y, mx.z};
   const unsigned mask = __activemask();
@@ -244,7 +299,10 @@ __device__ __forceinline__ void widened_box(F3 a, F3 b, F3 c, float inv_h, int b
 // (c (R + e) <= 1/4), and the right side grows slower than lb
 // (132 c (c2 R^2 + E0) <= 1/2); a sub-triangle that fails one (every
 // degenerate one does) is never culled (c2 = +inf).
-__device__ __forceinline__ void cull_coeffs(F3 ab, F3 ac, F3 cb, float R, float M, float& c2, float& E0) {
+// (c2 lb + E0 holds several times the bound derived above; with the conditions
+// met the denominator is off by less than 8 %, 188 / 0.92 < 256, so c2 / 4 and
+// the E1 that goes with it bound eps as well.)
+__device__ __forceinline__ void cull_coeffs(F3 ab, F3 ac, F3 cb, float R, float M, float& c2, float& E0, float& E1) {
   const float u = 5.9604645e-8f;
   const float e2 = fmaxf(dot3(ab, ab), fmaxf(dot3(ac, ac), dot3(cb, cb)));
   const float e = sqrtf(e2);
@@ -256,6 +314,7 @@ __device__ __forceinline__ void cull_coeffs(F3 ab, F3 ac, F3 cb, float R, float 
                   e0 < __int_as_float(0x7f800000);
   c2 = ok ? 2.0f * c : __int_as_float(0x7f800000);
   E0 = ok ? e0 : 0.0f;
+  E1 = ok ? e0 - 1.5f * c * e2 : 0.0f;
 }
 
 // A sub-triangle record: vertices, widened box, mesh, and the cull
@@ -272,57 +331,61 @@ __device__ __forceinline__ void put_subtri(SubTri* S, uint64_t idx, F3 a, F3 b, 
                                  max(abs(lo[2]), abs(hi[2]))) + 1);
   const float M = fmaxf(gm, fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(b.x))),
                                   fmaxf(fmaxf(fabsf(b.y), fabsf(b.z)), fmaxf(fmaxf(fabsf(c.x), fabsf(c.y)), fabsf(c.z)))));
-  float c2, e0;
-  cull_coeffs(sub3(b, a), sub3(c, a), sub3(c, b), R, M, c2, e0);
+  float c2, e0, e1;
+  cull_coeffs(sub3(b, a), sub3(c, a), sub3(c, b), R, M, c2, e0, e1);
   SubTri s;
   s.p0 = make_float4(a.x, a.y, a.z, b.x);
   s.p1 = make_float4(b.y, b.z, c.x, c.y);
-  s.p2 = make_float4(c.z, c2, e0, 0.f);
+  s.p2 = make_float4(c.z, c2, e0, e1);
   s.lo = make_int4(lo[0], lo[1], lo[2], mesh);
   s.hi = make_int4(hi[0], hi[1], hi[2], 0);
   S[idx] = s;
 }
 
-// mesh_to_volume.rs:75-116, same stepping and accumulation order.
+// mesh_to_volume.rs:75-116, same stepping and accumulation order, a thread per
+// sub-triangle: the running points are the start plus r steps down and k steps
+// along, added one at a time, so a thread repeats at most 2 n additions.  (A
+// thread per triangle took 5.1 ms on 810 triangles of about 11,000
+// sub-triangles each.)
 __global__ void k_subdivide(const float4* __restrict__ T, const uint32_t* __restrict__ nsub,
-                            const uint32_t* __restrict__ off, uint64_t nt, const MeshInfo* __restrict__ mi,
-                            const uint32_t* __restrict__ tri_base, int K, SubTri* __restrict__ S) {
-  uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
-  if (i >= nt || nsub[i] == 0) return;
+                            const uint32_t* __restrict__ off, uint64_t nt, uint64_t ns,
+                            const MeshInfo* __restrict__ mi, const uint32_t* __restrict__ tri_base, int K,
+                            SubTri* __restrict__ S) {
+  const uint64_t first = blockIdx.x * uint64_t(blockDim.x), o = first + threadIdx.x;
+  const uint64_t i = owner_of(off, nt, first, o);
+  if (o >= ns) return;
   const int mesh = find_seg(tri_base, K, i);
   const float h = mi[mesh].h, inv_h = mi[mesh].inv_h;
   const int band = mi[mesh].band;
-  float4 ta = T[3 * i], tb = T[3 * i + 1], tc = T[3 * i + 2];
-  F3 p1 = f3(ta.x, ta.y, ta.z), p2 = f3(tb.x, tb.y, tb.z), p3 = f3(tc.x, tc.y, tc.z);
-  uint64_t o = off[i];
+  const float4 ta = T[3 * i], tb = T[3 * i + 1], tc = T[3 * i + 2];
+  const F3 p1 = f3(ta.x, ta.y, ta.z), p2 = f3(tb.x, tb.y, tb.z), p3 = f3(tc.x, tc.y, tc.z);
   if (nsub[i] == 1) {
     put_subtri(S, o, p1, p2, p3, h, inv_h, band, mesh);
     return;
   }
   F3 e0 = sub3(p2, p1), e1 = sub3(p3, p1), e2 = sub3(p3, p2);
   float m = fmaxf(fmaxf(dot3(e0, e0), dot3(e1, e1)), dot3(e2, e2));
-  float ns = floorf(fdiv(fsqrt(m), h));
-  float inv = fdiv(1.0f, ns);
-  F3 s1 = scale3(sub3(p2, p1), inv);
-  F3 s2 = scale3(sub3(p3, p2), inv);
+  float ns_f = floorf(fdiv(fsqrt(m), h));
+  float inv = fdiv(1.0f, ns_f);
+  const F3 s1 = scale3(sub3(p2, p1), inv);
+  const F3 s2 = scale3(sub3(p3, p2), inv);
+  const uint32_t at = uint32_t(o - off[i]), r = isqrt(at), t = at - r * r;
   F3 a = p1;
-  uint32_t n = uint32_t(ns);
-  for (uint32_t r = 0; r < n; ++r) {
-    F3 b = add3(a, s1);
-    F3 c = add3(b, s2);
-    F3 a_s = add3(a, s2), b_s = add3(b, s2), c_s = add3(c, s2);
-    F3 a_prev = a;
-    for (uint32_t k = 0; k < r; ++k) {
-      put_subtri(S, o++, a_prev, b_s, a_s, h, inv_h, band, mesh);
-      put_subtri(S, o++, a_s, b_s, c_s, h, inv_h, band, mesh);
-      a_prev = a_s;
-      a_s = add3(a_s, s2);
-      b_s = add3(b_s, s2);
-      c_s = add3(c_s, s2);
-    }
-    put_subtri(S, o++, a, b, c, h, inv_h, band, mesh);
-    a = add3(a, s1);
+  for (uint32_t q = 0; q < r; ++q) a = add3(a, s1);
+  F3 b = add3(a, s1);
+  if (t == 2 * r) {  // the row's first upright sub-triangle comes last
+    put_subtri(S, o, a, b, add3(b, s2), h, inv_h, band, mesh);
+    return;
   }
+  const uint32_t k = t >> 1;
+  for (uint32_t q = 0; q < k; ++q) {
+    a = add3(a, s2);
+    b = add3(b, s2);
+  }
+  // a, b: column k of this row and the next
+  const F3 a1 = add3(a, s2), b1 = add3(b, s2);
+  if (t & 1u) put_subtri(S, o, a1, b1, add3(b1, s2), h, inv_h, band, mesh);
+  else put_subtri(S, o, a, b1, a1, h, inv_h, band, mesh);
 }
 
 // ------------------------------------------------- 2. brick directory -----
@@ -331,10 +394,10 @@ struct Dir {
   int dx, dy, dz;     // extent in bricks
 };
 
-__device__ __forceinline__ bool brick_range(const SubTri& s, const Dir& d, int lo[3], int hi[3]) {
-  lo[0] = (s.lo.x >> 3) - d.bx0; hi[0] = (s.hi.x >> 3) - d.bx0;
-  lo[1] = (s.lo.y >> 3) - d.by0; hi[1] = (s.hi.y >> 3) - d.by0;
-  lo[2] = (s.lo.z >> 3) - d.bz0; hi[2] = (s.hi.z >> 3) - d.bz0;
+__device__ __forceinline__ bool brick_range(int4 blo, int4 bhi, const Dir& d, int lo[3], int hi[3]) {
+  lo[0] = (blo.x >> 3) - d.bx0; hi[0] = (bhi.x >> 3) - d.bx0;
+  lo[1] = (blo.y >> 3) - d.by0; hi[1] = (bhi.y >> 3) - d.by0;
+  lo[2] = (blo.z >> 3) - d.bz0; hi[2] = (bhi.z >> 3) - d.bz0;
   return lo[0] >= 0 && lo[1] >= 0 && lo[2] >= 0 && hi[0] < d.dx && hi[1] < d.dy && hi[2] < d.dz;
 }
 
@@ -345,11 +408,11 @@ __device__ __forceinline__ bool brick_range(const SubTri& s, const Dir& d, int l
 // nearest to most of its voxels early and culls more of the rest (the result
 // does not depend on the order).  Integer arithmetic: count and fill agree.
 constexpr int LIST_CLASSES = 8;
-__device__ __forceinline__ int pair_class(const SubTri& s, int bx, int by, int bz) {
+__device__ __forceinline__ int pair_class(int4 lo, int4 hi, int bx, int by, int bz) {
   // twice the centre offset per axis, in voxels
-  const long long dx = (long long)s.lo.x + s.hi.x - (16LL * bx + 7);
-  const long long dy = (long long)s.lo.y + s.hi.y - (16LL * by + 7);
-  const long long dz = (long long)s.lo.z + s.hi.z - (16LL * bz + 7);
+  const long long dx = (long long)lo.x + hi.x - (16LL * bx + 7);
+  const long long dy = (long long)lo.y + hi.y - (16LL * by + 7);
+  const long long dz = (long long)lo.z + hi.z - (16LL * bz + 7);
   const long long q = 4 * (dx * dx + dy * dy + dz * dz);  // d >= 1.25 k  <=>  q >= 25 k^2
   int c = 0;
 #pragma unroll
@@ -366,7 +429,7 @@ __global__ void k_count_pairs(const SubTri* __restrict__ S, uint64_t ns, const D
   const Dir d = dirs[mesh];
   uint32_t* C = cnt + dir_base[mesh] * LIST_CLASSES;
   int lo[3], hi[3];
-  if (!brick_range(s, d, lo, hi)) {
+  if (!brick_range(s.lo, s.hi, d, lo, hi)) {
     atomicExch(&st[mesh].error, 2);
     return;
   }
@@ -374,7 +437,7 @@ __global__ void k_count_pairs(const SubTri* __restrict__ S, uint64_t ns, const D
     for (int y = lo[1]; y <= hi[1]; ++y)
       for (int z = lo[2]; z <= hi[2]; ++z)
         atomicAdd(&C[((uint64_t(x) * d.dy + y) * d.dz + z) * LIST_CLASSES +
-                     pair_class(s, x + d.bx0, y + d.by0, z + d.bz0)], 1u);
+                     pair_class(s.lo, s.hi, x + d.bx0, y + d.by0, z + d.bz0)], 1u);
   unsigned long long np = uint64_t(hi[0] - lo[0] + 1) * (hi[1] - lo[1] + 1) * (hi[2] - lo[2] + 1);
   unsigned long long vp = uint64_t(s.hi.x - s.lo.x + 1) * (s.hi.y - s.lo.y + 1) * (s.hi.z - s.lo.z + 1);
   warp_add(&st[mesh].n_pairs, np, mesh);
@@ -420,12 +483,12 @@ __global__ void k_fill_pairs(const SubTri* __restrict__ S, uint64_t ns, const Di
   const Dir d = dirs[mesh];
   uint32_t* C = cursor + dir_base[mesh] * LIST_CLASSES;
   int lo[3], hi[3];
-  if (!brick_range(s, d, lo, hi)) return;
+  if (!brick_range(s.lo, s.hi, d, lo, hi)) return;
   for (int x = lo[0]; x <= hi[0]; ++x)
     for (int y = lo[1]; y <= hi[1]; ++y)
       for (int z = lo[2]; z <= hi[2]; ++z) {
         uint32_t p = atomicAdd(&C[((uint64_t(x) * d.dy + y) * d.dz + z) * LIST_CLASSES +
-                                  pair_class(s, x + d.bx0, y + d.by0, z + d.bz0)], 1u);
+                                  pair_class(s.lo, s.hi, x + d.bx0, y + d.by0, z + d.bz0)], 1u);
         list[p] = uint32_t(i);
       }
 }
@@ -660,6 +723,12 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_brick_distance(
     if (lane == 0) masks[uint64_t(b) * 16 + warp + (THREADS / 32) * k] = m;
   }
 }
+
+}  // namespace bs
+
+#include "m2v_patch.cuh"
+
+namespace bs {
 
 // ------------------------------------------------- active voxel list ------
 __global__ void k_brick_popcount(const uint32_t* __restrict__ masks, uint64_t nb, uint32_t* __restrict__ cnt) {
@@ -1587,6 +1656,8 @@ bs_status exact_winding_numbers_impl(bs_ctx* ctx, const float* d_xyz, uint64_t n
 // ------------------------------------------------------------ driver ------
 static inline unsigned blocks(uint64_t n, unsigned t) { return unsigned((n + t - 1) / t); }
 
+constexpr double PATCH_PAIRS = 130.0;  // box pairs per band voxel from which the distance pass works on patches
+
 // One set of launches for a batch of meshes (the single-mesh call is a batch
 // of one).  Every kernel covers all meshes' triangles, bricks or voxels and
 // finds its mesh by a binary search of the per-mesh offsets; host syncs do
@@ -1880,8 +1951,8 @@ static std::vector<bs_volume*> batch_core(bs_ctx* ctx, const float* d_xyz, const
   }
 
   DBuf<float4> T(ctx, 3 * nt);
-  DBuf<uint32_t> nsub(ctx, nt + 1), soff(ctx, nt + 1);
-  BS_KERNEL(ctx, "k_gather", (k_gather<<<blocks(nt + 1, 256), 256, 0, s>>>(d_xyz, d_tri, nt, d_mi.p, d_tb.p, K, T.p, nsub.p, st.p)));
+  DBuf<uint32_t> nsub(ctx, nt + 1), soff(ctx, nt + 1), npat(ctx, nt + 1), poff;
+  BS_KERNEL(ctx, "k_gather", (k_gather<<<blocks(nt + 1, 256), 256, 0, s>>>(d_xyz, d_tri, nt, d_mi.p, d_tb.p, K, T.p, nsub.p, npat.p, st.p)));
   // the triangles, offsets and stats the tree build reads are ready here
   Event gathered, built;
   BS_CUDA(cudaEventRecord(gathered.e, s));
@@ -1920,14 +1991,43 @@ static std::vector<bs_volume*> batch_core(bs_ctx* ctx, const float* d_xyz, const
   BS_CUDA(cudaMemcpyAsync(d_db.p, dir_base.data(), (K + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, s));
 
   DBuf<SubTri> S(ctx, ns);
-  BS_KERNEL(ctx, "k_subdivide", (k_subdivide<<<blocks(nt, 128), 128, 0, s>>>(T.p, nsub.p, soff.p, nt, d_mi.p, d_tb.p, K, S.p)));
+  BS_KERNEL(ctx, "k_subdivide", (k_subdivide<<<blocks(ns, 128), 128, 0, s>>>(T.p, nsub.p, soff.p, nt, ns, d_mi.p, d_tb.p, K, S.p)));
+  // Patches pay where each band voxel lies in many sub-triangles' boxes: with
+  // d sub-triangles per squared voxel of surface (slender triangles: more) and
+  // boxes of about 2 band + 3.3 voxels, about 0.61 d (2 band + 3.3)^2 of them.
+  // Distance pass on sub-triangles / on patches at that many pairs per voxel:
+  // 41: 4.2 / 5.1 ms, 88: 5.6 / 6.0, 180: 3.44 / 3.31, 192: 15.6 / 12.2,
+  // 324: 12.9 / 7.8, 390: 18.9 / 11.4 (meshes of 0.8 k to 1 M triangles).
+  double est = 0.0, area = 0.0;
+  for (int m = 0; m < K; ++m) {
+    const double box = 2.0 * mi[m].band + 3.3;
+    est += 0.61 * box * box * double(hst[m].n_sub);
+    area += double(hst[m].area16) / 16.0;
+  }
+  const bool patches = area > 0.0 && est > PATCH_PAIRS * area && ns >= 2 * nt;
+  DBuf<Patch> pat;
+  uint64_t n_list = ns;  // entries of the lists' kind: sub-triangles or patches
+  if (patches) {
+    poff = DBuf<uint32_t>(ctx, nt + 1);
+    exclusive_scan(ctx, npat.p, poff.p, nt + 1);
+    uint32_t total_p = 0;
+    read_back(ctx, &total_p, poff.p + nt, sizeof(uint32_t));
+    n_list = total_p;
+    pat = DBuf<Patch>(ctx, n_list);
+    BS_KERNEL(ctx, "k_patches", (k_patches<<<blocks(n_list, 128), 128, 0, s>>>(T.p, nsub.p, soff.p, poff.p, nt, n_list, d_mi.p, S.p, pat.p, st.p)));
+    poff.reset();
+  }
+  npat.reset();
   nsub.reset();
   soff.reset();
 
   const uint64_t DC = D * LIST_CLASSES;
   DBuf<uint32_t> cnt(ctx, DC + 1), pair_off(ctx, DC + 1), flag(ctx, D + 1), bidx(ctx, D + 1);
   BS_CUDA(cudaMemsetAsync(cnt.p, 0, (DC + 1) * sizeof(uint32_t), s));
-  BS_KERNEL(ctx, "k_count_pairs", (k_count_pairs<<<blocks(ns, 256), 256, 0, s>>>(S.p, ns, d_dirs.p, d_db.p, cnt.p, st.p)));
+  if (patches)
+    BS_KERNEL(ctx, "k_count_pairs", (k_count_patches<<<blocks(n_list, 256), 256, 0, s>>>(pat.p, n_list, S.p, d_dirs.p, d_db.p, cnt.p, st.p)));
+  else
+    BS_KERNEL(ctx, "k_count_pairs", (k_count_pairs<<<blocks(ns, 256), 256, 0, s>>>(S.p, ns, d_dirs.p, d_db.p, cnt.p, st.p)));
   exclusive_scan(ctx, cnt.p, pair_off.p, DC + 1);
   BS_KERNEL(ctx, "k_dir_flags", (k_dir_flags<<<blocks(D + 1, 256), 256, 0, s>>>(pair_off.p, D, flag.p)));
   exclusive_scan(ctx, flag.p, bidx.p, D + 1);
@@ -1963,15 +2063,29 @@ static std::vector<bs_volume*> batch_core(bs_ctx* ctx, const float* d_xyz, const
     BS_CUDA(cudaMemcpyAsync(list_off.p + nb, pair_off.p + DC, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
     pair_off.reset();
     bidx.reset();
-    BS_KERNEL(ctx, "k_fill_pairs", (k_fill_pairs<<<blocks(ns, 256), 256, 0, s>>>(S.p, ns, d_dirs.p, d_db.p, cnt.p, list.p)));
+    if (patches)
+      BS_KERNEL(ctx, "k_fill_pairs", (k_fill_patches<<<blocks(n_list, 256), 256, 0, s>>>(pat.p, n_list, S.p, d_dirs.p, d_db.p, cnt.p, list.p)));
+    else
+      BS_KERNEL(ctx, "k_fill_pairs", (k_fill_pairs<<<blocks(ns, 256), 256, 0, s>>>(S.p, ns, d_dirs.p, d_db.p, cnt.p, list.p)));
     cnt.reset();
     const int dt = ctx->tune_dist_threads, db = ctx->tune_dist_batch;
-#define BS_DIST(TH, BA)                                                                                            \
+#define BS_DIST(TH, BA)                                                                                              \
   BS_KERNEL(ctx, "k_brick_distance", (k_brick_distance<TH, BA><<<unsigned(nb), TH, 0, s>>>(origins.p, list_off.p,  \
                                                                                             list.p, S.p, d_mi.p,     \
                                                                                             leaf_base.p, K, values.p, \
                                                                                             masks.p, st.p)))
-    if (dt == 64 && db == 8)
+#define BS_PATCH(TH)                                                                                                 \
+  BS_KERNEL(ctx, "k_brick_distance", (k_patch_distance<TH><<<unsigned(nb), TH, 0, s>>>(origins.p, list_off.p,      \
+                                                                                        list.p, pat.p, S.p, d_mi.p,  \
+                                                                                        leaf_base.p, K, values.p,    \
+                                                                                        masks.p, st.p)))
+    if (patches && dt == 64)
+      BS_PATCH(64);
+    else if (patches && dt == 256)
+      BS_PATCH(256);
+    else if (patches)
+      BS_PATCH(128);
+    else if (dt == 64 && db == 8)
       BS_DIST(64, 8);
     else if (dt == 64 && db == 32)
       BS_DIST(64, 32);
@@ -1988,8 +2102,10 @@ static std::vector<bs_volume*> batch_core(bs_ctx* ctx, const float* d_xyz, const
     else
       BS_DIST(128, 16);
 #undef BS_DIST
+#undef BS_PATCH
   }
   S.reset();
+  pat.reset();
 
   // active voxels, and per mesh its first brick / voxel
   // one tree per mesh over its original triangles, built on the side stream
