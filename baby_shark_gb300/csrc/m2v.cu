@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "bs_internal.cuh"
+#include "fast_sign.cuh"
 #include "ref_tree.cuh"
 
 namespace bs {
@@ -1375,7 +1376,7 @@ __device__ __forceinline__ float far3(const float4* __restrict__ c3, float rx, f
 // every lane takes the exact solid angle.  Node loads are warp-uniform, control
 // flow never diverges, and each lane's sum is at least as accurate as its own
 // traversal would be.  ORDER 3 adds the third-order far-field term.
-template <int ORDER>
+template <int ORDER, bool COUNT = true>
 __device__ __forceinline__ float wn_traverse(F3 q, const float4* __restrict__ inode, const float4* __restrict__ leaf,
                                              const float4* __restrict__ inode3, const float4* __restrict__ leaf3, int n,
                                              float beta, M2VStats* st, int (*stk)[WN_STACK]) {
@@ -1463,7 +1464,7 @@ __device__ __forceinline__ float wn_traverse(F3 q, const float4* __restrict__ in
   // flagged above, would drop some), takes a far field or an exact solid angle
   const uint32_t c_visit = (n > 1) ? 1u + 2u * uint32_t(it) : 1u;
   const uint32_t c_far = c_visit - c_exact - uint32_t(it);
-  if (lane == 0) {
+  if (COUNT && lane == 0) {
     atomicAdd(&st->wn_visits, (unsigned long long)c_visit);
     atomicAdd(&st->wn_far, (unsigned long long)c_far);
     atomicAdd(&st->wn_exact, (unsigned long long)c_exact);
@@ -1473,7 +1474,7 @@ __device__ __forceinline__ float wn_traverse(F3 q, const float4* __restrict__ in
 
 // Band voxel act[i] of the warp: its grid point and, after the traversal, the
 // sign of its distance (mesh_to_volume.rs:264-271).
-template <int ORDER>
+template <int ORDER, bool COUNT = true>
 __device__ __forceinline__ void wn_warp(const uint32_t* __restrict__ act, uint64_t i, bool valid, uint64_t last,
                                         const int4* __restrict__ origins, float* __restrict__ values,
                                         const float4* __restrict__ inode, const float4* __restrict__ leaf,
@@ -1484,7 +1485,7 @@ __device__ __forceinline__ void wn_warp(const uint32_t* __restrict__ act, uint64
   const int4 org = origins[b];
   const F3 q = f3(fmul(__int2float_rn(org.x + int(o >> 6)), h), fmul(__int2float_rn(org.y + int((o >> 3) & 7)), h),
                   fmul(__int2float_rn(org.z + int(o & 7)), h));
-  const float sum = wn_traverse<ORDER>(q, inode, leaf, inode3, leaf3, n, beta, st, stk);
+  const float sum = wn_traverse<ORDER, COUNT>(q, inode, leaf, inode3, leaf3, n, beta, st, stk);
   if (valid) {
     const float d = values[uint64_t(b) * 512 + o];
     values[uint64_t(b) * 512 + o] = (sum < thresh) ? copysignf(d, 1.0f) : copysignf(d, -1.0f);
@@ -1508,7 +1509,6 @@ __global__ void __launch_bounds__(32 * WARPS) k_wn_sign(const uint32_t* __restri
 
 // Batches: warps are numbered per mesh (warp_base[m] .. warp_base[m+1]) so
 // that a warp never holds voxels of two meshes.
-template <int ORDER>
 __global__ void __launch_bounds__(WN_THREADS) k_wn_sign_batch(const uint32_t* __restrict__ act,
                                                               const uint32_t* __restrict__ act_base,
                                                               const uint32_t* __restrict__ warp_base, int K,
@@ -1530,12 +1530,40 @@ __global__ void __launch_bounds__(WN_THREADS) k_wn_sign_batch(const uint32_t* __
   const uint64_t i = act_base[mesh] + (gw - warp_base[mesh]) * 32 + lane;
   const MeshInfo M = mi[mesh];
   const uint64_t ib = inode_base[mesh], lb = tri_base[mesh];
-  if (ORDER >= 3 && M.order >= 3)
+  if (M.order >= 3)
     wn_warp<3>(act, i, i < a1, a1 - 1, origins, values, inodes + 5 * ib, leaves + 5 * lb, inodes3 + 6 * ib,
                leaves3 + 6 * lb, int(M.n_tri), M.h, M.beta, M.thresh, stats + mesh, stk);
   else
     wn_warp<2>(act, i, i < a1, a1 - 1, origins, values, inodes + 5 * ib, leaves + 5 * lb, nullptr, nullptr,
                int(M.n_tri), M.h, M.beta, M.thresh, stats + mesh, stk);
+}
+
+// The warps that the filter (fast_sign.cu) did not settle: rest[0 .. *n_rest),
+// each by its first index into act.  They are few (0.2 % of a scan's) and
+// counted there.
+__global__ void __launch_bounds__(WN_THREADS) k_wn_sign_rest(const uint32_t* __restrict__ act,
+                                                             const uint32_t* __restrict__ act_base, int K,
+                                                             const MeshInfo* __restrict__ mi,
+                                                             const uint32_t* __restrict__ tri_base,
+                                                             const uint32_t* __restrict__ inode_base,
+                                                             const int4* __restrict__ origins,
+                                                             float* __restrict__ values,
+                                                             const float4* __restrict__ inodes,
+                                                             const float4* __restrict__ leaves, M2VStats* stats,
+                                                             const uint32_t* __restrict__ rest,
+                                                             const uint32_t* __restrict__ n_rest) {
+  __shared__ int stk[WN_WARPS][WN_STACK];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const uint32_t n = *n_rest;
+  for (uint32_t r = blockIdx.x * WN_WARPS + w; r < n; r += gridDim.x * WN_WARPS) {
+    const uint64_t i0 = rest[r], i = i0 + lane;
+    const int mesh = find_seg(act_base, K, i0);
+    const uint64_t a1 = act_base[mesh + 1];
+    const MeshInfo M = mi[mesh];
+    wn_warp<2, false>(act, i, i < a1, a1 - 1, origins, values, inodes + 5 * uint64_t(inode_base[mesh]),
+                      leaves + 5 * uint64_t(tri_base[mesh]), nullptr, nullptr, int(M.n_tri), M.h, M.beta, M.thresh,
+                      stats + mesh, stk);
+  }
 }
 
 // WindingNumbers::approximate (aabb_tree.rs:654-660) at arbitrary points: a
@@ -2114,7 +2142,8 @@ static std::vector<bs_volume*> batch_core(bs_ctx* ctx, const float* d_xyz, const
   // wn_tree 0: the reference's SAH tree, traversed per voxel in its summation
   // order (ref_tree.cu); 1: this library's PLOC tree, traversed per warp
   const bool ref_tree = params[size_t(which[0])].wn_tree == 0;
-  DBuf<float4> leaf, inode, leaf3, inode3;
+  DBuf<float4> leaf, inode, leaf3, inode3, frec;
+  DBuf<FastSignMesh> d_fm;
   RefTrees rt;
   {
     SideStream side(ctx);
@@ -2125,6 +2154,15 @@ static std::vector<bs_volume*> batch_core(bs_ctx* ctx, const float* d_xyz, const
       build_ref_trees(ctx, T.p, nt, K, tri_base.data(), betas, rt);
     } else {
       build_trees(ctx, T.p, nt, K, d_tb.p, d_ib.p, st.p, any3, leaf, inode, leaf3, inode3);
+      if (!any3) {
+        std::vector<FastSignMesh> fm(K);
+        for (int m = 0; m < K; ++m)
+          fm[m] = FastSignMesh{inode_base[m], tri_base[m], mi[m].n_tri, mi[m].h, mi[m].beta, mi[m].thresh};
+        d_fm = DBuf<FastSignMesh>(ctx, K);
+        BS_CUDA(cudaMemcpyAsync(d_fm.p, fm.data(), K * sizeof(FastSignMesh), cudaMemcpyHostToDevice, ctx->stream));
+        frec = DBuf<float4>(ctx, 4 * (2 * nt - uint64_t(K)));
+        fast_filter_records(ctx, inode.p, nt - uint64_t(K), d_ib.p, leaf.p, nt, d_tb.p, K, d_fm.p, frec.p);
+      }
     }
     BS_CUDA(cudaEventRecord(built.e, ctx->stream));
   }
@@ -2157,10 +2195,16 @@ static std::vector<bs_volume*> batch_core(bs_ctx* ctx, const float* d_xyz, const
   read_back(ctx, h_leaf_base.data(), leaf_base.p, (K + 1) * sizeof(uint32_t));
   read_back(ctx, h_act_base.data(), act_base.p, (K + 1) * sizeof(uint32_t));
   const uint64_t na = h_act_base[K];
-  std::vector<uint32_t> warp_base(K + 1, 0);
-  for (int m = 0; m < K; ++m) warp_base[m + 1] = warp_base[m] + (h_act_base[m + 1] - h_act_base[m] + 31) / 32;
-  DBuf<uint32_t> d_wb(ctx, K + 1);
-  BS_CUDA(cudaMemcpyAsync(d_wb.p, warp_base.data(), (K + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+  // per mesh its first warp, then its first span of the filter pass
+  std::vector<uint32_t> warp_base(2 * (K + 1), 0);
+  uint32_t* span_base = warp_base.data() + K + 1;
+  for (int m = 0; m < K; ++m) {
+    const uint32_t n_act = h_act_base[m + 1] - h_act_base[m];
+    warp_base[m + 1] = warp_base[m] + (n_act + 31) / 32;
+    span_base[m + 1] = span_base[m] + (n_act + FAST_SIGN_SPAN - 1) / FAST_SIGN_SPAN;
+  }
+  DBuf<uint32_t> d_wb(ctx, 2 * (K + 1));
+  BS_CUDA(cudaMemcpyAsync(d_wb.p, warp_base.data(), 2 * (K + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
   DBuf<uint32_t> act(ctx, std::max<uint64_t>(na, 1));
   if (nb) BS_KERNEL(ctx, "k_emit_active", (k_emit_active<<<blocks(nb * 32, 256), 256, 0, s>>>(masks.p, voff.p, nb, act.p)));
   vc.reset();
@@ -2181,34 +2225,35 @@ static std::vector<bs_volume*> batch_core(bs_ctx* ctx, const float* d_xyz, const
     if (rt_cnt[3]) fail(BS_ERR_CAPACITY, "winding-number traversal stack overflow");
   } else if (na > 0) {
     const uint64_t n_warps = warp_base[K];
-#define BS_WN1(O, WP, I3, L3)                                                                                   \
-  BS_KERNEL(ctx, "k_wn_sign", (k_wn_sign<O, WP><<<blocks(na, 32 * WP), 32 * WP, 0, s>>>(                      \
-                                  act.p, na, origins.p, values.p, inode.p, leaf.p, I3, L3, int(nt), mi[0].h,   \
-                                  mi[0].beta, mi[0].thresh, st.p)))
+#define BS_WN3(WP)                                                                                              \
+  BS_KERNEL(ctx, "k_wn_sign", (k_wn_sign<3, WP><<<blocks(na, 32 * WP), 32 * WP, 0, s>>>(                      \
+                                  act.p, na, origins.p, values.p, inode.p, leaf.p, inode3.p, leaf3.p, int(nt), \
+                                  mi[0].h, mi[0].beta, mi[0].thresh, st.p)))
     const int ww = ctx->tune_wn_warps;
-    if (K == 1 && mi[0].order < 3) {
-      if (ww == 2)
-        BS_WN1(2, 2, nullptr, nullptr);
-      else if (ww == 8)
-        BS_WN1(2, 8, nullptr, nullptr);
-      else
-        BS_WN1(2, 4, nullptr, nullptr);
+    if (!any3) {
+      DBuf<uint32_t> rest(ctx, n_warps + 1);  // listed warps, and their number
+      BS_CUDA(cudaMemsetAsync(rest.p + n_warps, 0, sizeof(uint32_t), s));
+      static_assert(offsetof(M2VStats, wn_exact) == offsetof(M2VStats, wn_visits) + 16 && sizeof(M2VStats) % 8 == 0,
+                    "the filter adds to three consecutive counters");
+      fast_sign(ctx, act.p, act_base.p, d_wb.p + K + 1, span_base[K], K, d_fm.p, origins.p, values.p, frec.p,
+                nt - uint64_t(K), inode.p, leaf.p, rest.p, rest.p + n_warps, &st.p->wn_visits,
+                uint32_t(sizeof(M2VStats) / 8));
+      const unsigned grid = unsigned(std::min<uint64_t>(blocks(n_warps, WN_WARPS), uint64_t(8 * 152)));
+      BS_KERNEL(ctx, "k_wn_sign_rest", (k_wn_sign_rest<<<grid, WN_THREADS, 0, s>>>(act.p, act_base.p, K, d_mi.p, d_tb.p, d_ib.p, origins.p,
+                                                                               values.p, inode.p, leaf.p, st.p, rest.p, rest.p + n_warps)));
     } else if (K == 1) {
       if (ww == 2)
-        BS_WN1(3, 2, inode3.p, leaf3.p);
+        BS_WN3(2);
       else if (ww == 8)
-        BS_WN1(3, 8, inode3.p, leaf3.p);
+        BS_WN3(8);
       else
-        BS_WN1(3, 4, inode3.p, leaf3.p);
-    } else if (!any3)
-      BS_KERNEL(ctx, "k_wn_sign", (k_wn_sign_batch<2><<<blocks(n_warps, WN_WARPS), WN_THREADS, 0, s>>>(act.p, act_base.p, d_wb.p, K, d_mi.p, d_tb.p,
-                                                                                       d_ib.p, origins.p, values.p, inode.p, leaf.p,
-                                                                                       nullptr, nullptr, st.p)));
-    else
-      BS_KERNEL(ctx, "k_wn_sign", (k_wn_sign_batch<3><<<blocks(n_warps, WN_WARPS), WN_THREADS, 0, s>>>(act.p, act_base.p, d_wb.p, K, d_mi.p, d_tb.p,
+        BS_WN3(4);
+    } else {
+      BS_KERNEL(ctx, "k_wn_sign", (k_wn_sign_batch<<<blocks(n_warps, WN_WARPS), WN_THREADS, 0, s>>>(act.p, act_base.p, d_wb.p, K, d_mi.p, d_tb.p,
                                                                                        d_ib.p, origins.p, values.p, inode.p, leaf.p,
                                                                                        inode3.p, leaf3.p, st.p)));
-#undef BS_WN1
+    }
+#undef BS_WN3
   }
   read_back(ctx, hst.data(), st.p, K * sizeof(M2VStats));
   uint64_t n_vp = 0, n_p = 0, visits = 0, far = 0, exact = 0, n_ev = 0;
