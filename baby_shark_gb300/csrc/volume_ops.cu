@@ -81,11 +81,6 @@ __global__ void k_assign_children(const uint32_t* __restrict__ child_sorted, con
   }
 }
 
-__global__ void k_fill_f(float* p, uint64_t n, float v) {
-  uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
-  if (i < n) p[i] = v;
-}
-
 // Groups `n` children (origins) into parent nodes of level `lv`.
 static void build_level(bs_ctx* ctx, const int4* child_org, uint64_t n, Level& lv) {
   cudaStream_t s = ctx->stream;
@@ -106,10 +101,9 @@ static void build_level(bs_ctx* ctx, const int4* child_org, uint64_t n, Level& l
   read_back(ctx, &ng, gidx.p + n, sizeof(uint32_t));
   lv.alloc(ctx, ng);
   BS_CUDA(cudaMemsetAsync(lv.d_state, 0xff, ng * uint64_t(lv.slots) * sizeof(int), s));
-  BS_KERNEL(ctx, "k_fill_f", (k_fill_f<<<nblk(ng * uint64_t(lv.slots), 256), 256, 0, s>>>(lv.d_tile, ng * uint64_t(lv.slots), 0.0f)));
+  BS_CUDA(cudaMemsetAsync(lv.d_tile, 0, ng * uint64_t(lv.slots) * sizeof(float), s));
   BS_KERNEL(ctx, "k_assign_children", (k_assign_children<<<nblk(n, 256), 256, 0, s>>>(v2.p, flag.p, gidx.p, n, child_org, lv.log2,
                                                                           lv.child_shift, lv.d_state, lv.d_key)));
-  lv.sync_keys(ctx);
 }
 
 void Level::alloc(bs_ctx* ctx, uint64_t count) {
@@ -141,12 +135,190 @@ void Level::sync_keys(bs_ctx* ctx) {
   }
 }
 
+// Both levels at once where the L1 nodes' bounding box has at most NODE_CELLS
+// cells: a cell per node in (x, y, z) order, ranked by one block, gives the
+// same nodes in the same order as sorting the leaves' node keys, in four small
+// launches and one host read.  Volumes spread wider take build_level.  The
+// subtraction of two volumes of 32 k leaves took 2.06 ms with the sorts and a
+// read of every level's count and keys, 1.48 ms with this, one read of the
+// result's counts and k_ff_internal's masks.
+constexpr int NODE_CELLS = 1 << 16, NODE2_CELLS = 2048, NODE2_KEYS = 8;
+struct NodeBounds {
+  int lo[3], neg_hi[3];  // L1 node coordinates, by atomicMin
+  int n1, n2;            // nodes of both levels; n1 < 0: too many cells
+  int4 key2[NODE2_KEYS]; // the first L2 nodes
+};
+struct NodeBox {  // cells of L1 nodes and of the L2 nodes around them
+  int x, y, z, dx, dy, dz, x2, y2, z2, ex, ey, ez;
+  long long cells, cells2;
+};
+__device__ __forceinline__ NodeBox node_box(const NodeBounds& b) {
+  NodeBox q;
+  q.x = b.lo[0];
+  q.y = b.lo[1];
+  q.z = b.lo[2];
+  q.dx = 1 - b.neg_hi[0] - q.x;
+  q.dy = 1 - b.neg_hi[1] - q.y;
+  q.dz = 1 - b.neg_hi[2] - q.z;
+  q.x2 = q.x >> L2_LOG2;
+  q.y2 = q.y >> L2_LOG2;
+  q.z2 = q.z >> L2_LOG2;
+  q.ex = (-b.neg_hi[0] >> L2_LOG2) - q.x2 + 1;
+  q.ey = (-b.neg_hi[1] >> L2_LOG2) - q.y2 + 1;
+  q.ez = (-b.neg_hi[2] >> L2_LOG2) - q.z2 + 1;
+  q.cells = (long long)q.dx * q.dy * q.dz;
+  q.cells2 = (long long)q.ex * q.ey * q.ez;
+  return q;
+}
+__device__ __forceinline__ bool box_fits(const NodeBox& q) { return q.cells <= NODE_CELLS && q.cells2 <= NODE2_CELLS; }
+__device__ __forceinline__ int node_cell(const NodeBox& q, int4 o) {
+  return (((o.x >> L2_CHILD_SHIFT) - q.x) * q.dy + (o.y >> L2_CHILD_SHIFT) - q.y) * q.dz + (o.z >> L2_CHILD_SHIFT) - q.z;
+}
+
+__global__ void k_node_bounds(const int4* __restrict__ org, uint64_t n, NodeBounds* __restrict__ b) {
+  const uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
+  const int4 o = org[i < n ? i : n - 1];
+  const int c[3] = {o.x >> L2_CHILD_SHIFT, o.y >> L2_CHILD_SHIFT, o.z >> L2_CHILD_SHIFT};
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int lo = __reduce_min_sync(0xffffffffu, c[k]), hi = __reduce_max_sync(0xffffffffu, c[k]);
+    if ((threadIdx.x & 31) == 0) {
+      if (lo < b->lo[k]) atomicMin(&b->lo[k], lo);
+      if (-hi < b->neg_hi[k]) atomicMin(&b->neg_hi[k], -hi);
+    }
+  }
+}
+
+__global__ void k_node_mark(const int4* __restrict__ org, uint64_t n, const NodeBounds* __restrict__ b,
+                            int* __restrict__ cell) {
+  const uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
+  const NodeBox q = node_box(*b);
+  if (i < n && box_fits(q)) cell[node_cell(q, org[i])] = 1;
+}
+
+// One block: cell[c] = rank of the L1 node there, key1[rank] = its origin;
+// cell2 / key2 likewise for the L2 nodes.
+__global__ void __launch_bounds__(1024) k_node_rank(NodeBounds* __restrict__ b, int* __restrict__ cell,
+                                                    int4* __restrict__ key1, uint64_t max_nodes,
+                                                    int* __restrict__ cell2) {
+  __shared__ int mark2[NODE2_CELLS], sums[32], base;
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const NodeBox q = node_box(*b);
+  if (!box_fits(q)) {
+    if (t == 0) b->n1 = -1;
+    return;
+  }
+  for (int c = t; c < NODE2_CELLS; c += 1024) mark2[c] = 0;
+  // rank of a set cell among 1024 at a time, after `base`
+  auto rank = [&](bool on) {
+    const unsigned m = __ballot_sync(0xffffffffu, on);
+    if (lane == 0) sums[w] = __popc(m);
+    __syncthreads();
+    int r = base + __popc(m & ((1u << lane) - 1u)), total = 0;
+    for (int k = 0; k < 32; ++k) {
+      if (k < w) r += sums[k];
+      total += sums[k];
+    }
+    __syncthreads();
+    if (t == 0) base += total;
+    __syncthreads();
+    return r;
+  };
+  if (t == 0) base = 0;
+  __syncthreads();
+  for (int c0 = 0; c0 < int(q.cells); c0 += 1024) {
+    const int c = c0 + t;
+    const bool on = c < int(q.cells) && cell[c] != 0;
+    const int r = rank(on);
+    if (on && uint64_t(r) < max_nodes) {
+      cell[c] = r;
+      const int x = q.x + c / (q.dy * q.dz), y = q.y + c / q.dz % q.dy, z = q.z + c % q.dz;
+      key1[r] = make_int4(x << L2_CHILD_SHIFT, y << L2_CHILD_SHIFT, z << L2_CHILD_SHIFT, 0);
+      mark2[(((x >> L2_LOG2) - q.x2) * q.ey + (y >> L2_LOG2) - q.y2) * q.ez + (z >> L2_LOG2) - q.z2] = 1;
+    }
+  }
+  __syncthreads();
+  if (t == 0) {
+    b->n1 = base;
+    base = 0;
+  }
+  __syncthreads();
+  for (int c0 = 0; c0 < int(q.cells2); c0 += 1024) {
+    const int c = c0 + t;
+    const bool on = c < int(q.cells2) && mark2[c] != 0;
+    const int r = rank(on);
+    if (on) {
+      cell2[c] = r;
+      if (r < NODE2_KEYS)
+        b->key2[r] = make_int4((q.x2 + c / (q.ey * q.ez)) << L2_SHIFT, (q.y2 + c / q.ez % q.ey) << L2_SHIFT,
+                               (q.z2 + c % q.ez) << L2_SHIFT, 0);
+    }
+  }
+  if (t == 0) b->n2 = base;
+}
+
+// Children into their slots; the L2 nodes' keys by their children (all write
+// the same).
+__global__ void k_node_fill(const int4* __restrict__ org, uint64_t n, const NodeBounds* __restrict__ b,
+                            const int* __restrict__ cell, const int* __restrict__ cell2,
+                            const int4* __restrict__ key_in, int4* __restrict__ key1, int* __restrict__ state1,
+                            int4* __restrict__ key2, int* __restrict__ state2) {
+  const uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
+  const NodeBox q = node_box(*b);
+  auto slot = [](int4 o, int log2, int shift) {
+    const int m = (1 << log2) - 1;
+    return (((o.x >> shift) & m) << (2 * log2)) | (((o.y >> shift) & m) << log2) | ((o.z >> shift) & m);
+  };
+  if (i < n) {
+    const int4 o = org[i];
+    state1[uint64_t(cell[node_cell(q, o)]) * L1_SLOTS + slot(o, L1_LOG2, L1_CHILD_SHIFT)] = int(i);
+  }
+  if (i < uint64_t(b->n1)) {
+    const int4 k = key_in[i];
+    key1[i] = k;
+    const int g = cell2[(((k.x >> L2_SHIFT) - q.x2) * q.ey + (k.y >> L2_SHIFT) - q.y2) * q.ez + (k.z >> L2_SHIFT) - q.z2];
+    state2[uint64_t(g) * L2_SLOTS + slot(k, L2_LOG2, L2_CHILD_SHIFT)] = int(i);
+    key2[g] = make_int4((k.x >> L2_SHIFT) << L2_SHIFT, (k.y >> L2_SHIFT) << L2_SHIFT, (k.z >> L2_SHIFT) << L2_SHIFT, 0);
+  }
+}
+
+// Returns false (nothing built) when the box has too many cells.
+static bool build_levels(bs_ctx* ctx, const int4* org, uint64_t n, Level& l1, Level& l2) {
+  cudaStream_t s = ctx->stream;
+  DBuf<NodeBounds> b(ctx, 1);
+  const uint64_t max1 = std::min<uint64_t>(n, NODE_CELLS);
+  DBuf<int> cell(ctx, NODE_CELLS), cell2(ctx, NODE2_CELLS);
+  DBuf<int4> key(ctx, max1);
+  BS_CUDA(cudaMemsetAsync(b.p, 0x7f, sizeof(NodeBounds), s));
+  BS_CUDA(cudaMemsetAsync(cell.p, 0, NODE_CELLS * sizeof(int), s));
+  BS_KERNEL(ctx, "k_node_bounds", (k_node_bounds<<<nblk(n, 256), 256, 0, s>>>(org, n, b.p)));
+  BS_KERNEL(ctx, "k_node_mark", (k_node_mark<<<nblk(n, 256), 256, 0, s>>>(org, n, b.p, cell.p)));
+  BS_KERNEL(ctx, "k_node_rank", (k_node_rank<<<1, 1024, 0, s>>>(b.p, cell.p, key.p, max1, cell2.p)));
+  NodeBounds h;
+  read_back(ctx, &h, b.p, sizeof h);
+  if (h.n1 < 0) return false;
+  l1.alloc(ctx, uint64_t(h.n1));
+  l2.alloc(ctx, uint64_t(h.n2));
+  for (Level* lv : {&l1, &l2}) {
+    BS_CUDA(cudaMemsetAsync(lv->d_state, 0xff, lv->n * uint64_t(lv->slots) * sizeof(int), s));
+    BS_CUDA(cudaMemsetAsync(lv->d_tile, 0, lv->n * uint64_t(lv->slots) * sizeof(float), s));
+  }
+  BS_KERNEL(ctx, "k_node_fill", (k_node_fill<<<nblk(n, 256), 256, 0, s>>>(org, n, b.p, cell.p, cell2.p, key.p, l1.d_key, l1.d_state,
+                                                                      l2.d_key, l2.d_state)));
+  if (h.n2 <= NODE2_KEYS) l2.h_key.assign(h.key2, h.key2 + h.n2);
+  else l2.sync_keys(ctx);
+  return true;
+}
+
 Upper* ensure_upper(bs_ctx* ctx, bs_volume* v) {
   if (v->upper) return v->upper;
   Upper* u = new Upper();
   try {
-    build_level(ctx, v->d_origins, v->n_leaves, u->l1);
-    build_level(ctx, u->l1.d_key, u->l1.n, u->l2);
+    if (v->n_leaves && !build_levels(ctx, v->d_origins, v->n_leaves, u->l1, u->l2)) {
+      build_level(ctx, v->d_origins, v->n_leaves, u->l1);
+      build_level(ctx, u->l1.d_key, u->l1.n, u->l2);
+      u->l2.sync_keys(ctx);
+    }
   } catch (...) {
     u->l1.free(ctx);
     u->l2.free(ctx);
@@ -263,28 +435,49 @@ __global__ void __launch_bounds__(32 * FF_WARPS) k_ff_leaf(float* __restrict__ v
   }
 }
 
-// internal_node/flood_fill.rs:17-117 for one node per CTA, one thread per z-line.
+// internal_node/flood_fill.rs:17-117 for one node per CTA.  The slots are read
+// once, coalesced: per z-line a word of shared memory each for the present
+// slots and for the signs they carry (a tile's own, a branch's last value),
+// from which one thread per line carries the sign through the empty slots, as
+// k_ff_leaf does.  63 us for the one L2 node of a volume with the slots read
+// again along every carry, 30 us here.
 template <int LOG2>
-__global__ void k_ff_internal(int* __restrict__ state, float* __restrict__ tile, uint64_t n,
+__global__ void k_ff_internal(const int* __restrict__ state, float* __restrict__ tile, uint64_t n,
                               const uint8_t* __restrict__ cfirst, const uint8_t* __restrict__ clast,
                               uint8_t* __restrict__ first_neg, uint8_t* __restrict__ last_neg) {
-  constexpr int DIM = 1 << LOG2, S = DIM * DIM * DIM;
+  constexpr int DIM = 1 << LOG2, LINES = DIM * DIM, S = DIM * LINES;
   const uint64_t node = blockIdx.x;
   if (node >= n) return;
-  int* st = state + node * S;
+  const int* st = state + node * S;
   float* tl = tile + node * S;
+  __shared__ uint32_t there[LINES], minus[LINES];  // bit z of line x DIM + y; minus: later the fill
   __shared__ int s_first_tile, s_first_branch, s_any_none;
+  const int lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     s_first_tile = S;
     s_first_branch = S;
     s_any_none = 0;
   }
   __syncthreads();
+  // blockDim is a multiple of 32 and S of blockDim
+#pragma unroll 4
   for (int o = threadIdx.x; o < S; o += blockDim.x) {
     const int q = st[o];
-    if (q == -2) atomicMin(&s_first_tile, o);
-    else if (q >= 0) atomicMin(&s_first_branch, o);
-    if (q != -2) s_any_none = 1;  // value_mask not full
+    const bool on = q >= 0 || q == -2;
+    const bool neg = q >= 0 ? clast[q] != 0 : (q == -2 && signbit(tl[o]));
+    const unsigned m_on = __ballot_sync(0xffffffffu, on), m_neg = __ballot_sync(0xffffffffu, neg);
+    const unsigned m_tile = __ballot_sync(0xffffffffu, q == -2), m_branch = __ballot_sync(0xffffffffu, q >= 0);
+    const int z0 = lane & ~(DIM - 1);  // 32 slots are one line (32) or two (16)
+    if (lane == z0) {
+      const uint32_t keep = DIM == 32 ? 0xffffffffu : 0xffffu;
+      there[o >> LOG2] = (m_on >> z0) & keep;
+      minus[o >> LOG2] = (m_neg >> z0) & keep;
+    }
+    if (lane == 0) {
+      if (m_tile) atomicMin(&s_first_tile, o + __ffs(m_tile) - 1);
+      if (m_branch) atomicMin(&s_first_branch, o + __ffs(m_branch) - 1);
+      if (m_tile != 0xffffffffu) s_any_none = 1;  // value_mask not full
+    }
   }
   __syncthreads();
   const int fv = s_first_tile, fb = s_first_branch;
@@ -292,24 +485,32 @@ __global__ void k_ff_internal(int* __restrict__ state, float* __restrict__ tile,
     bool i0;
     if (fv < S && (fb >= S || fv <= fb)) i0 = signbit(tl[fv]);
     else i0 = cfirst[st[fb]] != 0;
-    // carry sign of a present slot: tile -> its sign, branch -> child's last value sign
-    auto carry = [&](int o, bool& c) {
-      const int q = st[o];
-      if (q >= 0) c = clast[q] != 0;
-      else if (q == -2) c = signbit(tl[o]);
-    };
-    for (int line = threadIdx.x; line < DIM * DIM; line += blockDim.x) {
+    uint32_t fill[(LINES + 255) / 256];
+    int k = 0;
+    for (int line = threadIdx.x; line < LINES; line += blockDim.x, ++k) {
       const int x = line / DIM, y = line % DIM;
-      bool c = i0;
-      for (int xx = 0; xx <= x; ++xx) carry(xx * DIM * DIM, c);
-      for (int yy = 0; yy <= y; ++yy) carry(x * DIM * DIM + yy * DIM, c);
+      uint32_t c = i0;
+      for (int xx = 0; xx <= x; ++xx)
+        if (there[xx * DIM] & 1u) c = minus[xx * DIM] & 1u;
+      for (int yy = 0; yy <= y; ++yy)
+        if (there[x * DIM + yy] & 1u) c = minus[x * DIM + yy] & 1u;
+      const uint32_t on = there[line], sg = minus[line];
+      uint32_t f = 0;
+#pragma unroll
       for (int z = 0; z < DIM; ++z) {
-        const int o = x * DIM * DIM + y * DIM + z;
-        if (st[o] == -1)
-          tl[o] = signed_far(c);
-        else
-          carry(o, c);
+        if ((on >> z) & 1u) c = (sg >> z) & 1u;
+        else f |= c << z;
       }
+      fill[k] = f;
+    }
+    __syncthreads();
+    k = 0;
+    for (int line = threadIdx.x; line < LINES; line += blockDim.x, ++k) minus[line] = fill[k];
+    __syncthreads();
+#pragma unroll 4
+    for (int o = threadIdx.x; o < S; o += blockDim.x) {
+      const int line = o >> LOG2, z = o & (DIM - 1);
+      if (!((there[line] >> z) & 1u)) tl[o] = signed_far((minus[line] >> z) & 1u);
     }
   }
   __syncthreads();
@@ -455,8 +656,8 @@ template <int LOG2>
 __global__ void k_csg_slots(int op, const Req* __restrict__ plan, uint64_t n_out, const int* __restrict__ sa_,
                             const float* __restrict__ ta_, const int* __restrict__ sb_, const float* __restrict__ tb_,
                             int* __restrict__ out_state, float* __restrict__ out_tile, Req* __restrict__ child_req,
-                            uint32_t* __restrict__ child_flag) {
-  constexpr int S = 1 << (3 * LOG2);
+                            uint32_t* __restrict__ child_flag, unsigned long long* __restrict__ n_tiles) {
+  constexpr int S = 1 << (3 * LOG2);  // a multiple of the block: whole warps leave below
   const uint64_t e = blockIdx.y;
   const int o = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n_out || o >= S) return;
@@ -505,6 +706,8 @@ __global__ void k_csg_slots(int op, const Req* __restrict__ plan, uint64_t n_out
     }
   }
   if (cr.type >= 0) st = 0;  // placeholder; rewritten with the output child index
+  const unsigned tiles = __ballot_sync(0xffffffffu, st == -2);
+  if (tiles && (threadIdx.x & 31) == 0) atomicAdd(n_tiles, (unsigned long long)__popc(tiles));
   out_state[io] = st;
   out_tile[io] = tv;
   child_req[io] = cr;
@@ -650,7 +853,7 @@ void refresh_tiles(bs_ctx* ctx, bs_volume* v) {
 // Output slots of one level and the requests for the level below.
 template <int LOG2>
 static uint64_t csg_level(bs_ctx* ctx, int op, const DBuf<Req>& plan, uint64_t n_out, const Level& A, const Level& B,
-                          Level& out, DBuf<Req>& child_plan) {
+                          Level& out, DBuf<Req>& child_plan, unsigned long long* n_tiles) {
   constexpr uint64_t S = 1ull << (3 * LOG2);
   cudaStream_t s = ctx->stream;
   out.alloc(ctx, n_out);
@@ -664,7 +867,7 @@ static uint64_t csg_level(bs_ctx* ctx, int op, const DBuf<Req>& plan, uint64_t n
   BS_CUDA(cudaMemsetAsync(flag.p + n, 0, sizeof(uint32_t), s));
   dim3 g(unsigned((S + 255) / 256), unsigned(n_out));
   BS_KERNEL(ctx, "k_csg_slots", (k_csg_slots<LOG2><<<g, 256, 0, s>>>(op, plan.p, n_out, A.d_state, A.d_tile, B.d_state, B.d_tile,
-                                                         out.d_state, out.d_tile, req.p, flag.p)));
+                                                         out.d_state, out.d_tile, req.p, flag.p, n_tiles)));
   scan_excl(ctx, flag.p, pos.p, n + 1);
   uint32_t nc = 0;
   read_back(ctx, &nc, pos.p + n, sizeof(uint32_t));
@@ -715,10 +918,11 @@ bs_volume* volume_csg_impl(bs_ctx* ctx, bs_volume* a, bs_volume* b, int op) {
     if (!plan2.empty())
       BS_CUDA(cudaMemcpyAsync(d_plan2.p, plan2.data(), plan2.size() * sizeof(Req), cudaMemcpyHostToDevice, ctx->stream));
     DBuf<Req> plan1, plan0;
-    const uint64_t n1 = csg_level<L2_LOG2>(ctx, op, d_plan2, plan2.size(), ua->l2, ub->l2, uo->l2, plan1);
-    const uint64_t n0 = csg_level<L1_LOG2>(ctx, op, plan1, n1, ua->l1, ub->l1, uo->l1, plan0);
-    uo->l2.sync_keys(ctx);
-    uo->l1.sync_keys(ctx);
+    DBuf<unsigned long long> cnt(ctx, 2);  // active voxels, active tiles
+    BS_CUDA(cudaMemsetAsync(cnt.p, 0, 2 * sizeof(unsigned long long), ctx->stream));
+    const uint64_t n1 = csg_level<L2_LOG2>(ctx, op, d_plan2, plan2.size(), ua->l2, ub->l2, uo->l2, plan1, cnt.p + 1);
+    const uint64_t n0 = csg_level<L1_LOG2>(ctx, op, plan1, n1, ua->l1, ub->l1, uo->l1, plan0, cnt.p + 1);
+    for (const Req& r : plan2) uo->l2.h_key.push_back(r.type == 1 ? ub->l2.h_key[size_t(r.b)] : ua->l2.h_key[size_t(r.a)]);
     // union never empties a merged node: a merged slot's A side was a branch,
     // which stays a branch or becomes an active inside tile
     out->n_leaves = n0;
@@ -730,14 +934,12 @@ bs_volume* volume_csg_impl(bs_ctx* ctx, bs_volume* a, bs_volume* b, int op) {
                                                                             a->d_masks, b->d_origins, b->d_values,
                                                                             b->d_masks, out->d_origins, out->d_values,
                                                                             out->d_masks)));
-    DBuf<unsigned long long> cnt(ctx, 1);
-    BS_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(unsigned long long), ctx->stream));
     if (n0)
       BS_KERNEL(ctx, "k_count_active", (k_count_active<<<nblk(n0 * 16, 256), 256, 0, ctx->stream>>>(out->d_masks, n0, cnt.p)));
-    unsigned long long na = 0;
-    read_back(ctx, &na, cnt.p, sizeof(na));
-    out->n_active = na;
-    refresh_tiles(ctx, out);
+    unsigned long long c[2];
+    read_back(ctx, c, cnt.p, sizeof c);
+    out->n_active = c[0];
+    if (c[1]) refresh_tiles(ctx, out);
   } catch (...) {
     delete out;
     throw;
