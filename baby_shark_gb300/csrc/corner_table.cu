@@ -14,15 +14,35 @@
 
 #include <algorithm>
 #include <cstring>
+#include <memory>
+#include <utility>
 
 #include "bs_internal.cuh"
 
+// Host arrays that are sized first and then filled by copies from the device:
+// resize leaves new elements as they are (zeroing 19 MB cost 0.33 ms).
+template <class T>
+struct Unset : std::allocator<T> {
+  template <class U>
+  struct rebind {
+    using other = Unset<U>;
+  };
+  template <class U>
+  void construct(U* p) {
+    ::new (static_cast<void*>(p)) U;
+  }
+  template <class U, class... A>
+  void construct(U* p, A&&... a) {
+    ::new (static_cast<void*>(p)) U(std::forward<A>(a)...);
+  }
+};
+
 struct bs_corner_table {
-  std::vector<float> pos;             // [slots][3]
-  std::vector<uint8_t> deleted;       // [slots]
-  std::vector<int32_t> vcorner;       // [slots] -1 none
-  std::vector<int32_t> cvertex;       // [corners]
-  std::vector<int32_t> copp;          // [corners] -1 none
+  std::vector<float, Unset<float>> pos;         // [slots][3]
+  std::vector<uint8_t, Unset<uint8_t>> deleted; // [slots]
+  std::vector<int32_t, Unset<int32_t>> vcorner; // [slots] -1 none
+  std::vector<int32_t, Unset<int32_t>> cvertex; // [corners]
+  std::vector<int32_t, Unset<int32_t>> copp;    // [corners] -1 none
 };
 
 namespace bs {
