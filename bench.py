@@ -60,7 +60,6 @@ H = 0.002
 BAND = 3
 # Algorithmic work per unit, counted from the reference's operations.
 FLOP_PER_PAIR = 84          # closest point + norm, triangle3.rs:317-382 (face-region path)
-CULL_FLOP_PER_PAIR = 20     # voxel to bounding box distance and the cull comparison
 WN_FLOP_FAR = 31            # far test + order-1/2 terms, aabb_tree.rs:662-671, 803-816
 WN_FLOP_EXACT = 70          # Van Oosterom-Strackee solid angle, aabb_tree.rs:582-615 (atan2 as 20)
 WN_FAR_PER_VOXEL = 141.46   # the oracle's traversal of the reference's SAH tree over the whole torus
@@ -68,15 +67,14 @@ WN_EXACT_PER_VOXEL = 14.96  # (1,048,576 triangles) from the 4.5 M band voxels o
 #                             counts per band voxel (oracle/traversal_counts.py)
 WN_FLOP_PER_VOXEL = int(round(WN_FAR_PER_VOXEL * WN_FLOP_FAR + WN_EXACT_PER_VOXEL * WN_FLOP_EXACT))
 # dram__bytes_read.sum + dram__bytes_write.sum per launch from one ncu capture of
-# the half-ring case (k_wn_sign 322 MB for 17,900,503 band voxels,
-# k_brick_distance 716 MB for 3,416,413,115 voxel pairs), scaled to a full
-# torus by the units processed (35,669,277 voxels; 6,848,421,294 pairs);
-# k_rt_sign captured on one full torus (582.8 MB read + 272.0 MB written)
-TRAFFIC_PER_LAUNCH = {"k_wn_sign": 642e6, "k_brick_distance": 1436e6, "k_rt_sign": 854.8e6}
-# smsp__inst_executed.sum per launch of the same capture of k_rt_sign (one
-# full torus, 35,669,277 band voxels): warp instructions, the kernel's real
-# bound (it issues on 86 % of the cycles); scaled by the voxels of a launch
-RT_SIGN_WARP_INST_PER_VOXEL = 67.74e9 / 35669277
+# one full torus (35,589,878 band voxels: k_rt_sign 526 + 167 MB, the distance
+# pass on patches 1,168 + 266 MB) and of a scan with holes (14,745,700 band
+# voxels: the fast tree's pass 399 + 70 MB, scaled by the voxels)
+TRAFFIC_PER_LAUNCH = {"k_wn_sign": 1134e6, "k_brick_distance": 1433e6, "k_rt_sign": 693e6}
+# smsp__inst_executed.sum per launch of the same capture of k_rt_sign: warp
+# instructions, the kernel's real bound (it issues on 70 % of the cycles);
+# scaled by the voxels of a launch
+RT_SIGN_WARP_INST_PER_VOXEL = 13.23e9 / 35589878
 SM_COUNT_GB300 = 152
 SCHEDULERS_PER_SM = 4
 METRIC = "band voxels/s mesh→SDF+sign: learned/batched vs plain GPU, 0 sign flips"
@@ -400,18 +398,15 @@ def run_ours(args):
     extra = {}
     if name == "k_brick_distance":
         ev = stats["voxel_pairs_evaluated"]
-        flops = FLOP_PER_PAIR * ev + CULL_FLOP_PER_PAIR * stats["voxel_pairs"]
-        algo = ("%d FLOP x %d evaluated (voxel, sub-triangle) pairs + %d FLOP cull test x %d pairs per launch"
-                % (FLOP_PER_PAIR, ev, CULL_FLOP_PER_PAIR, stats["voxel_pairs"]))
+        # the culls are per patch and sub-triangle where patches are used: not counted
+        flops = FLOP_PER_PAIR * ev
+        algo = "%d FLOP x %d evaluated (voxel, sub-triangle) pairs per launch" % (FLOP_PER_PAIR, ev)
         extra["reference_equivalent_tflops"] = FLOP_PER_PAIR * stats["voxel_pairs"] / per_launch_s / 1e12
         extra["pairs_evaluated_fraction"] = ev / max(1, stats["voxel_pairs"])
     elif name == "k_rt_sign":
         flops = WN_FLOP_PER_VOXEL * stats["active_voxels"]
-        # one traversal per voxel of the reference's own tree: the executed
-        # far-field and exact counts are the reference's (per voxel)
-        executed = WN_FLOP_FAR * stats["wn_far"] + WN_FLOP_EXACT * stats["wn_exact"]
-        extra["executed_tflops"] = executed / per_launch_s / 1e12
-        extra["executed_flop_per_launch"] = executed
+        # the far fields and triangles of the voxels' own cuts are the reference's;
+        # the filter evaluates most of them once for many voxels
         extra["far_per_voxel"] = stats["wn_far"] / max(1, stats["active_voxels"])
         extra["exact_per_voxel"] = stats["wn_exact"] / max(1, stats["active_voxels"])
         algo = ("%d FLOP per band voxel (the reference's own traversal: %.0f far-field nodes x %d FLOP + "
@@ -430,11 +425,6 @@ def run_ours(args):
                           "voxel; peak = 152 SMs x 4 schedulers x the sampled SM clock"}
     elif name == "k_wn_sign":
         flops = WN_FLOP_PER_VOXEL * stats["active_voxels"]
-        # what the warp-coherent traversal executes: every lane of a warp evaluates
-        # each node the warp takes as far, and each leaf the warp opens exactly
-        executed = 32 * (WN_FLOP_FAR * stats["wn_warp_far"] + WN_FLOP_EXACT * stats["wn_warp_exact"])
-        extra["executed_tflops"] = executed / per_launch_s / 1e12
-        extra["executed_flop_per_launch"] = executed
         algo = ("%d FLOP per band voxel (the reference's own traversal: %.0f far-field nodes x %d FLOP + "
                 "%.0f exact triangles x %d FLOP, counted by the oracle) x %d voxels per launch"
                 % (WN_FLOP_PER_VOXEL, WN_FAR_PER_VOXEL, WN_FLOP_FAR, WN_EXACT_PER_VOXEL, WN_FLOP_EXACT,
