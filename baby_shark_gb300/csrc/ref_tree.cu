@@ -51,7 +51,12 @@ constexpr int NB = 12;                 // buckets per axis (aabb_tree.rs:437)
 constexpr uint32_t MIN_LEAF = 3;       // with_min_objects_per_leaf(3) (aabb_tree.rs:640)
 constexpr int MAX_DEPTH = 40;          // AABBTree's default max depth (aabb_tree.rs:69)
 constexpr uint32_t SMALL = 512;        // nodes up to this many triangles are finished by one CTA
-constexpr uint32_t CHUNK = 2048;       // positions per block in the passes over large nodes
+// Positions per block in the passes over large nodes.  Few, so that the passes
+// fill the SMs: k_rt_place took 0.214 ms for the nine levels of 81,920 triangles
+// with 2048 a block, 0.107 ms with 512 (256: 0.103 ms); 1.11 and 0.95 ms for the
+// thirteen levels of 1.2 M.  More from 4 M triangles on, where the thread that
+// lists a node's chunks would write thousands.
+constexpr uint32_t CHUNK_FEW = 512, CHUNK_MANY = 2048, CHUNK_MANY_FROM = 1u << 22;
 constexpr int BKW = 3 * NB * 7;        // bins of a node: axis x bucket x (count, lo xyz, hi xyz)
 constexpr int STACK = MAX_DEPTH;       // pending left sums of a traversal
 constexpr int ST_THREADS = 256;        // CTA of the small-node kernel
@@ -102,8 +107,9 @@ struct RtBuild {  // device arrays the kernels share
   uint32_t* leaf_prio;
   RtSeg* big_next;
   RtSeg* small;
-  uint32_t* counters;  // [0] next large nodes, [1] small nodes, [2] error
-  uint32_t cap_big, cap_small;
+  RtChunk* chunks_next;
+  uint32_t* counters;  // [0] next large nodes, [1] their chunks, [2] error, [3] large leaves, [4] small nodes
+  uint32_t cap_big, cap_small, cap_chunks, chunk;
 };
 
 // Axis list after a stable sort along axis a: a first, then the earlier axes
@@ -235,13 +241,21 @@ __device__ void place(const RtBuild& B, const RtSeg& c) {
   if (c.count <= MIN_LEAF || c.depth >= MAX_DEPTH) {
     emit_leaf(B, c.first, c.count, c.prio, c.parent, c.side);
   } else if (c.count <= SMALL) {
-    const uint32_t s = atomicAdd(&B.counters[1], 1u);
+    const uint32_t s = atomicAdd(&B.counters[4], 1u);
     if (s < B.cap_small) B.small[s] = c;
     else atomicExch(&B.counters[2], 1u);
   } else {
     const uint32_t s = atomicAdd(&B.counters[0], 1u);
-    if (s < B.cap_big) B.big_next[s] = c;
-    else atomicExch(&B.counters[2], 1u);
+    const uint32_t n = (c.count + B.chunk - 1) / B.chunk, at = atomicAdd(&B.counters[1], n);
+    if (s < B.cap_big && at < B.cap_chunks && n <= B.cap_chunks - at) {
+      B.big_next[s] = c;
+      for (uint32_t k = 0; k < n; ++k) {
+        const uint32_t b = c.first + k * B.chunk;
+        B.chunks_next[at + k] = RtChunk{s, b, min(b + B.chunk, c.first + c.count)};
+      }
+    } else {
+      atomicExch(&B.counters[2], 1u);
+    }
   }
 }
 
@@ -1199,8 +1213,11 @@ void build_ref_trees(bs_ctx* ctx, const float4* T, uint64_t nt, int K, const uin
   const uint32_t cap_big = uint32_t(nt / SMALL + K + 1), cap_small = uint32_t(nt / 4 + K + 1);
   DBuf<RtSeg> big[2] = {DBuf<RtSeg>(ctx, cap_big), DBuf<RtSeg>(ctx, cap_big)};
   DBuf<RtSeg> small(ctx, cap_small);
-  DBuf<uint32_t> counters(ctx, 4);
-  BS_CUDA(cudaMemsetAsync(counters.p, 0, 4 * sizeof(uint32_t), s));
+  const uint32_t chunk = nt < CHUNK_MANY_FROM ? CHUNK_FEW : CHUNK_MANY;
+  const uint32_t cap_chunks = uint32_t(nt / chunk) + cap_big;  // every node's last one may be short
+  DBuf<RtChunk> chunks[2] = {DBuf<RtChunk>(ctx, cap_chunks), DBuf<RtChunk>(ctx, cap_chunks)};
+  DBuf<uint32_t> counters(ctx, 5);
+  BS_CUDA(cudaMemsetAsync(counters.p, 0, 5 * sizeof(uint32_t), s));
   RtBuild B;
   B.obA = obA.p;
   B.obB = obB.p;
@@ -1216,40 +1233,37 @@ void build_ref_trees(bs_ctx* ctx, const float4* T, uint64_t nt, int K, const uin
   B.counters = counters.p;
   B.cap_big = cap_big;
   B.cap_small = cap_small;
+  B.cap_chunks = cap_chunks;
+  B.chunk = chunk;
   int cur = 0;
   B.big_next = big[cur].p;
+  B.chunks_next = chunks[cur].p;
   BS_KERNEL(ctx, "k_rt_roots", (k_rt_roots<<<nblk(K, 128), 128, 0, s>>>(B, d_tb.p, K, mb.p)));
-  uint32_t hc[4];
+  uint32_t hc[5];
   read_back(ctx, hc, counters.p, sizeof hc);
   uint32_t n_cur = hc[0];
-  std::vector<RtSeg> hs;
+  // per level one host read: the nodes come with the chunks of their passes
   for (int level = 0; n_cur > 0; ++level) {
     if (level > MAX_DEPTH || hc[2]) fail(BS_ERR_CAPACITY, "reference tree build: node lists overflowed");
-    hs.resize(n_cur);
-    read_back(ctx, hs.data(), big[cur].p, n_cur * sizeof(RtSeg));
-    std::vector<RtChunk> chunks;
-    for (uint32_t k = 0; k < n_cur; ++k)
-      for (uint32_t b0 = hs[k].first; b0 < hs[k].first + hs[k].count; b0 += CHUNK)
-        chunks.push_back(RtChunk{k, b0, std::min(b0 + CHUNK, hs[k].first + hs[k].count)});
-    const uint32_t nch = uint32_t(chunks.size());
-    DBuf<RtChunk> d_ch(ctx, nch);
-    BS_CUDA(cudaMemcpyAsync(d_ch.p, chunks.data(), nch * sizeof(RtChunk), cudaMemcpyHostToDevice, s));
+    const uint32_t nch = hc[1];
+    const RtChunk* d_ch = chunks[cur].p;
     DBuf<uint32_t> bk(ctx, uint64_t(n_cur) * BKW), cb(ctx, 24 * uint64_t(n_cur)), cursor(ctx, 2 * uint64_t(n_cur));
     DBuf<RtDec> dec(ctx, n_cur);
     BS_KERNEL(ctx, "k_rt_bins_init", (k_rt_bins_init<<<nblk(uint64_t(n_cur) * BKW, 256), 256, 0, s>>>(bk.p, uint64_t(n_cur) * BKW)));
-    BS_KERNEL(ctx, "k_rt_bins", (k_rt_bins<<<nch, 256, 0, s>>>(d_ch.p, big[cur].p, perm.p, obA.p, obB.p, obC.p, bk.p)));
+    BS_KERNEL(ctx, "k_rt_bins", (k_rt_bins<<<nch, 256, 0, s>>>(d_ch, big[cur].p, perm.p, obA.p, obB.p, obC.p, bk.p)));
     BS_KERNEL(ctx, "k_rt_decide", (k_rt_decide<<<nblk(n_cur, 128), 128, 0, s>>>(big[cur].p, n_cur, bk.p, dec.p, cb.p, cursor.p)));
-    BS_KERNEL(ctx, "k_rt_place", (k_rt_place<<<nch, 256, 0, s>>>(d_ch.p, big[cur].p, dec.p, perm.p, ptmp.p, obA.p, obB.p, obC.p, cb.p, cursor.p)));
-    BS_KERNEL(ctx, "k_rt_copyback", (k_rt_copyback<<<nch, 256, 0, s>>>(d_ch.p, dec.p, ptmp.p, perm.p)));
-    BS_CUDA(cudaMemsetAsync(counters.p, 0, sizeof(uint32_t), s));
+    BS_KERNEL(ctx, "k_rt_place", (k_rt_place<<<nch, 256, 0, s>>>(d_ch, big[cur].p, dec.p, perm.p, ptmp.p, obA.p, obB.p, obC.p, cb.p, cursor.p)));
+    BS_KERNEL(ctx, "k_rt_copyback", (k_rt_copyback<<<nch, 256, 0, s>>>(d_ch, dec.p, ptmp.p, perm.p)));
+    BS_CUDA(cudaMemsetAsync(counters.p, 0, 2 * sizeof(uint32_t), s));
     B.big_next = big[cur ^ 1].p;
+    B.chunks_next = chunks[cur ^ 1].p;
     BS_KERNEL(ctx, "k_rt_children", (k_rt_children<<<nblk(n_cur, 128), 128, 0, s>>>(B, big[cur].p, n_cur, dec.p, cb.p, cursor.p)));
     read_back(ctx, hc, counters.p, sizeof hc);
     n_cur = hc[0];
     cur ^= 1;
   }
   if (hc[2]) fail(BS_ERR_CAPACITY, "reference tree build: node lists overflowed");
-  const uint32_t n_small = hc[1];
+  const uint32_t n_small = hc[4];
   if (n_small) BS_KERNEL(ctx, "k_rt_small", (k_rt_small<<<n_small, ST_THREADS, 0, s>>>(B)));
   DBuf<uint32_t> big_leaves(ctx, nt / (LEAF_SORT_THREAD + 1) + 1);
   BS_KERNEL(ctx, "k_rt_leaf_sort", (k_rt_leaf_sort<<<nblk(nt, 256), 256, 0, s>>>(nt, out.leaf_cnt.p, leaf_prio.p, perm.p, obA.p, obB.p, obC.p,
