@@ -130,12 +130,13 @@ __global__ void __launch_bounds__(32 * COPY_WARPS) k_gather_leaves(
 // --------------------------------------------------------------- sweeps ----
 // fast_sweep.rs:509-537, operation for operation.
 __device__ __forceinline__ float compute_distance(float a1, float a2, float a3, float h) {
-  // ascending (all are finite and not negative)
-  const float lo = fminf(a1, a3), hi = fmaxf(a1, a3);
-  a1 = fminf(lo, a2);
-  a3 = fmaxf(lo, a2);
-  a2 = fminf(a3, hi);
-  a3 = fmaxf(a3, hi);
+  // utils.rs:5-17, comparing and swapping as there: a NaN (from_fn keeps NaN
+  // voxels) moves like any value that is not greater and makes the distance
+  // NaN, which no voxel takes; fminf and fmaxf would drop it
+  float t;
+  if (a1 > a3) { t = a1; a1 = a3; a3 = t; }
+  if (a1 > a2) { t = a1; a1 = a2; a2 = t; }
+  if (a2 > a3) { t = a2; a2 = a3; a3 = t; }
   const float s1 = fadd(a1, h);
   if (fabsf(s1) <= a2) return s1;
   const float a1a2_sum = fadd(a1, a2);
