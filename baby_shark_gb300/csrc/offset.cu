@@ -131,8 +131,8 @@ __global__ void __launch_bounds__(32 * COPY_WARPS) k_gather_leaves(
 // fast_sweep.rs:509-537, operation for operation.
 __device__ __forceinline__ float compute_distance(float a1, float a2, float a3, float h) {
   // utils.rs:5-17, comparing and swapping as there: a NaN (from_fn keeps NaN
-  // voxels) moves like any value that is not greater and makes the distance
-  // NaN, which no voxel takes; fminf and fmaxf would drop it
+  // voxels) stays where it is met, and a distance that needs it is NaN, which
+  // no voxel takes; fminf and fmaxf would drop it
   float t;
   if (a1 > a3) { t = a1; a1 = a3; a3 = t; }
   if (a1 > a2) { t = a1; a1 = a2; a2 = t; }
@@ -219,8 +219,12 @@ __device__ __forceinline__ int face_pad(int ax, int fl, int i) {
 }
 
 // option_min_by with the |.| comparison of fast_sweep.rs:141-144, a the + side;
-// an inactive neighbour is +inf (active values are finite), so "none" stays +inf.
-__device__ __forceinline__ float min_by_abs(float a, float b) { return (fabsf(a) > fabsf(b)) ? b : a; }
+// an inactive neighbour is +inf (active values are not: remove_if drops them),
+// so "none" stays +inf.  A NaN is not greater than anything, but it comes
+// before "none", which the second comparison is for.
+__device__ __forceinline__ float min_by_abs(float a, float b) {
+  return (fabsf(a) > fabsf(b) || a == INFINITY) ? b : a;
+}
 
 // fast_sweep.rs:125-183 for the voxel at padded index p of the tile W: the
 // distance it is offered, +inf where none is.  It takes it when it is below

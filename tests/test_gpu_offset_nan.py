@@ -14,8 +14,8 @@ from tests.gpu_common import as_dict, context, unpack_mask
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("share", [0.001])
-@pytest.mark.parametrize("d", [0.13, -0.13])
+@pytest.mark.parametrize("share", [0.001, 0.02, 0.3])
+@pytest.mark.parametrize("d", [0.13, -0.13, 0.4])
 def test_nan_voxels_match_oracle(share, d):
     h, n = np.float32(0.1), 24
     rng = np.random.default_rng(int(1000 * share))
