@@ -6,8 +6,8 @@
 // needs only the side of the threshold its sum lies on
 // (mesh_to_volume.rs:264-271).  This pass walks the same cut and evaluates it
 // in cheaper arithmetic with a bound on how far the traversal's float32 sum
-// can be (sign_filter.cuh); the warps whose cut or whose voxels' sides it
-// cannot settle are listed and traversed (k_wn_sign_rest), so the signs are
+// can be (sign_filter.cuh); the warps whose voxels' sides it cannot settle, or
+// whose cut it has no room for, are listed and traversed (k_wn_sign_rest), so the signs are
 // the traversal's.
 //
 // What makes it cheap: nodes are tested 32 at a time, one per lane, against
@@ -29,7 +29,8 @@ constexpr int FRONT = 448;   // nodes a warp's first phase leaves to its groups
 constexpr int STACK = 256;   // pending nodes
 constexpr float E_GROUP = 0.02f;  // truncation error of one expanded node in a group's first attempt
 constexpr int SLOT = 5;      // float4 per lane's broadcast slot: 4 and one that keeps the banks apart
-constexpr float TAU_LO = 0.999999f, TAU_HI = 1.000001f;  // the float32 squared distances are within 4 u
+// the float32 squared distances are within 4 u: outside of this the traversal's test is certain
+constexpr float TAU_LO = 0.999999f, TAU_HI = 1.000001f;
 
 __device__ __forceinline__ int segment(const uint32_t* __restrict__ base, int K, uint32_t i) {
   int lo = 0, hi = K - 1;
@@ -106,8 +107,8 @@ __global__ void __launch_bounds__(32 * WARPS, 24 / WARPS) k_wn_filter(
     const uint32_t* __restrict__ act, const uint32_t* __restrict__ act_base, const uint32_t* __restrict__ span_base,
     int K, const FastSignMesh* __restrict__ meshes, const int4* __restrict__ origins, float* __restrict__ values,
     const float4* __restrict__ frec0, uint64_t ni, const float4* __restrict__ inode, const float4* __restrict__ leaf0,
-    uint32_t* __restrict__ rest, uint32_t* __restrict__ n_rest, unsigned long long* __restrict__ counts,
-    uint32_t count_stride) {
+    uint32_t* __restrict__ rest, uint32_t n_warps, uint32_t* __restrict__ n_rest,
+    unsigned long long* __restrict__ counts, uint32_t count_stride) {
   __shared__ FastSmem smem[WARPS];
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
@@ -153,16 +154,19 @@ __global__ void __launch_bounds__(32 * WARPS, 24 / WARPS) k_wn_filter(
   const float reach = Proot.w + (fabsf(Proot.x - bcx) + fabsf(Proot.y - bcy) + fabsf(Proot.z - bcz)) + brho;
   const bool in_range = reach * reach < R2_MAX;  // false for NaN
   const uint32_t n_groups = (nv + 31) / 32;
-  uint32_t c_visit = 0, c_far = 0, c_exact = 0;  // per lane, but visits per warp
+  // Work of the groups whose cut was walked to its end.  Every visit opens a
+  // node, takes its far field or its solid angle, and opening gives two more:
+  // (visits + 1) / 2 of a cut are not openings.
+  uint32_t c_visit = 0, c_cuts = 0, c_exact = 0;
 
   // ---- first phase, all voxels of the span ----
   int* stk = sm.stack;
   int n_front = 0;
+  uint32_t n_shared = 0;  // visits of every group's cut in this phase
   {
     Taylor TB;
     taylor_clear(TB);
     int sp = 1;
-    uint32_t n_far = 0, n_open = 0;
     bool over = false;
     if (lane == 0) stk[0] = root;
     __syncwarp();
@@ -186,8 +190,7 @@ __global__ void __launch_bounds__(32 * WARPS, 24 / WARPS) k_wn_filter(
       }
       const bool keep = have && !expand && !open;
       const unsigned m_o = __ballot_sync(FULLM, open), m_f = __ballot_sync(FULLM, keep);
-      n_far += __popc(__ballot_sync(FULLM, expand));
-      n_open += __popc(m_o);
+      n_shared += __popc(__ballot_sync(FULLM, expand || open));
       if (n_front + __popc(m_f) > FRONT || sp + 2 * __popc(m_o) > STACK) {
         over = true;
         break;
@@ -204,7 +207,7 @@ __global__ void __launch_bounds__(32 * WARPS, 24 / WARPS) k_wn_filter(
     }
     if (over) {  // no room: every group starts at the root
       taylor_clear(TB);
-      n_far = n_open = 0;
+      n_shared = 0;
       n_front = 1;
       if (lane == 0) sm.front[0] = root;
     }
@@ -215,8 +218,6 @@ __global__ void __launch_bounds__(32 * WARPS, 24 / WARPS) k_wn_filter(
       if (lane == 0) sm.taylor[k] = TB.c[k];
     }
     __syncwarp();
-    if (lane == 0) c_far += n_far * n_groups;
-    c_visit += (n_far + n_open) * n_groups;
   }
 
   // ---- groups: the traversal's 32 voxels ----
@@ -236,6 +237,7 @@ __global__ void __launch_bounds__(32 * WARPS, 24 / WARPS) k_wn_filter(
     const float rho =
         sqrtf(__uint_as_float(__reduce_max_sync(FULLM, __float_as_uint(dx * dx + dy * dy + dz * dz)))) * 1.00001f;
     unsigned open_lanes = __ballot_sync(FULLM, ok);  // voxels without a sign yet
+    bool counted = false;
     // first with the span's polynomial and frontier; the voxels this does not
     // settle once more from the root with a finer bound
     for (int attempt = 0; attempt < 2; ++attempt) {
@@ -245,8 +247,8 @@ __global__ void __launch_bounds__(32 * WARPS, 24 / WARPS) k_wn_filter(
       Lane s;
       s.w = s.mag = s.etri = 0.0f;
       s.bad = !in_range;
-      uint32_t n_add = 0;
-      bool lost = false;  // the cut itself is not settled, or has no room
+      uint32_t n_add = 0, n_visit = 0, n_exact = 0;
+      bool lost = false;  // no room for the cut
       int sp = 0, pos = 0;
       if (attempt) {
         if (lane == 0) stk[0] = root;
@@ -298,9 +300,15 @@ __global__ void __launch_bounds__(32 * WARPS, 24 / WARPS) k_wn_filter(
             r2min = fminf(r2min, ex * ex + ey * ey + ez * ez);
           }
         }
-        const bool near = r2min <= tau_lo;
-        lost |= __any_sync(FULLM, mixed && !near && !(r2min >= tau_hi)) != 0;
-        if (lost) break;
+        bool near = r2min <= tau_lo;
+        // too close to call, or a NaN: the traversal's own comparison
+        for (unsigned m = __ballot_sync(FULLM, mixed && !near && !(r2min >= tau_hi)); m; m &= m - 1u) {
+          const int src = __ffs(m) - 1;
+          const float hx = __shfl_sync(FULLM, H.x, src), hy = __shfl_sync(FULLM, H.y, src),
+                      hz = __shfl_sync(FULLM, H.z, src), hw = __shfl_sync(FULLM, H.w, src);
+          const bool opens = !__all_sync(FULLM, cut_dist2(hx - q.x, hy - q.y, hz - q.z) > hw);
+          if (lane == src) near = opens;
+        }
         if (mixed) far = !near;
         const bool direct = far && !t.poly;
         if (far) {
@@ -327,11 +335,7 @@ __global__ void __launch_bounds__(32 * WARPS, 24 / WARPS) k_wn_filter(
         }
         const bool tri = have && !far && ref < 0, open = have && !far && ref >= 0;
         const unsigned m_o = __ballot_sync(FULLM, open);
-        if (attempt == 0) {
-          c_visit += n;
-          c_far += far;
-          c_exact += tri;
-        }
+        n_visit += n;
         if (sp + 2 * __popc(m_o) > STACK) {
           lost = true;
           break;
@@ -342,7 +346,9 @@ __global__ void __launch_bounds__(32 * WARPS, 24 / WARPS) k_wn_filter(
           stk[at + 1] = right;
         }
         sp += 2 * __popc(m_o);
-        for (unsigned m = __ballot_sync(FULLM, tri); m; m &= m - 1u) {
+        unsigned m = __ballot_sync(FULLM, tri);
+        n_exact += __popc(m);
+        for (; m; m &= m - 1u) {
           const float4* L = leaf + 5 * uint64_t(~__shfl_sync(FULLM, ref, __ffs(m) - 1)) + 2;
           const float4 A = __ldg(L), B = __ldg(L + 1), C = __ldg(L + 2);
           ++n_add;
@@ -364,6 +370,12 @@ __global__ void __launch_bounds__(32 * WARPS, 24 / WARPS) k_wn_filter(
         for (int d = 16; d > 0; d >>= 1) T.c[k] += __shfl_xor_sync(FULLM, T.c[k], d);
       }
       float W = s.w + taylor_at(T.c, dx, dy, dz), mag = s.mag + T.c[10], err = T.c[9];
+      if (attempt == 0 && !lost) {
+        c_visit += n_visit + n_shared;
+        ++c_cuts;
+        c_exact += n_exact;
+        counted = true;
+      }
       if (attempt == 0) {
         W += taylor_at(sm.taylor, q.x - bcx, q.y - bcy, q.z - bcz);
         err += sm.taylor[9];
@@ -383,15 +395,15 @@ __global__ void __launch_bounds__(32 * WARPS, 24 / WARPS) k_wn_filter(
       open_lanes = __ballot_sync(FULLM, mine && !settled);
       if (!open_lanes || lost) break;
     }
-    if (open_lanes && lane == 0) rest[atomicAdd(n_rest, 1u)] = i0 + 32 * g;
+    if (open_lanes && lane == 0)
+      rest[counted ? atomicAdd(n_rest, 1u) : n_warps - 1u - atomicAdd(n_rest + 1, 1u)] = i0 + 32 * g;
     __syncwarp();
   }
-  const uint32_t far_all = __reduce_add_sync(FULLM, c_far), exact_all = __reduce_add_sync(FULLM, c_exact);
   if (lane == 0) {
     unsigned long long* c = counts + uint64_t(mesh) * count_stride;
     atomicAdd(c, (unsigned long long)c_visit);
-    atomicAdd(c + 1, (unsigned long long)far_all);
-    atomicAdd(c + 2, (unsigned long long)exact_all);
+    atomicAdd(c + 1, (unsigned long long)((c_visit + c_cuts) / 2 - c_exact));
+    atomicAdd(c + 2, (unsigned long long)c_exact);
   }
 }
 
@@ -408,13 +420,12 @@ void fast_filter_records(bs_ctx* ctx, const float4* inode, uint64_t n_internal, 
 void fast_sign(bs_ctx* ctx, const uint32_t* act, const uint32_t* d_act_base, const uint32_t* d_span_base,
                uint32_t n_spans, int K, const FastSignMesh* d_meshes, const int4* origins, float* values,
                const float4* frec, uint64_t n_internal, const float4* inode, const float4* leaf, uint32_t* rest,
-               uint32_t* n_rest, unsigned long long* d_counts, uint32_t count_stride) {
+               uint32_t n_warps, uint32_t* n_rest, unsigned long long* d_counts, uint32_t count_stride) {
   if (n_spans == 0) return;
 #define BS_WN_FILTER(W)                                                                                            \
   BS_KERNEL(ctx, "k_wn_sign", (k_wn_filter<W><<<(n_spans + W - 1) / W, 32 * W, 0, ctx->stream>>>(                                \
                                   act, d_act_base, d_span_base, K, d_meshes, origins, values, frec, n_internal,    \
-                                  inode, leaf, rest, n_rest, d_counts,             \
-                                  count_stride)))
+                                  inode, leaf, rest, n_warps, n_rest, d_counts, count_stride)))
   if (ctx->tune_wn_warps == 2)
     BS_WN_FILTER(2);
   else if (ctx->tune_wn_warps == 8)

@@ -1376,10 +1376,11 @@ __device__ __forceinline__ float far3(const float4* __restrict__ c3, float rx, f
 // every lane takes the exact solid angle.  Node loads are warp-uniform, control
 // flow never diverges, and each lane's sum is at least as accurate as its own
 // traversal would be.  ORDER 3 adds the third-order far-field term.
-template <int ORDER, bool COUNT = true>
+// `count`: whether its work is added to st.
+template <int ORDER>
 __device__ __forceinline__ float wn_traverse(F3 q, const float4* __restrict__ inode, const float4* __restrict__ leaf,
                                              const float4* __restrict__ inode3, const float4* __restrict__ leaf3, int n,
-                                             float beta, M2VStats* st, int (*stk)[WN_STACK]) {
+                                             float beta, M2VStats* st, int (*stk)[WN_STACK], bool count = true) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const float beta2 = beta * beta;
   float sum = 0.f, comp = 0.f;  // Kahan-compensated accumulation
@@ -1393,7 +1394,7 @@ __device__ __forceinline__ float wn_traverse(F3 q, const float4* __restrict__ in
     if (node >= 0) {
       const float4 P = inode[5 * node];
       const float rx = P.x - q.x, ry = P.y - q.y, rz = P.z - q.z;
-      const float r2 = rx * rx + ry * ry + rz * rz;
+      const float r2 = cut_dist2(rx, ry, rz);
       if (!__all_sync(0xffffffffu, r2 > P.w * P.w * beta2)) return true;
       const float4 A = inode[5 * node + 1], B0 = inode[5 * node + 2], B1 = inode[5 * node + 3],
                    B2 = inode[5 * node + 4];
@@ -1414,7 +1415,7 @@ __device__ __forceinline__ float wn_traverse(F3 q, const float4* __restrict__ in
     const int li = ~node;
     const float4 P = leaf[5 * li];
     const float rx = P.x - q.x, ry = P.y - q.y, rz = P.z - q.z;
-    const float r2 = rx * rx + ry * ry + rz * rz;
+    const float r2 = cut_dist2(rx, ry, rz);
     float wv;
     if (__all_sync(0xffffffffu, r2 > P.w * P.w * beta2)) {
       const float4 A = leaf[5 * li + 1];
@@ -1464,7 +1465,7 @@ __device__ __forceinline__ float wn_traverse(F3 q, const float4* __restrict__ in
   // flagged above, would drop some), takes a far field or an exact solid angle
   const uint32_t c_visit = (n > 1) ? 1u + 2u * uint32_t(it) : 1u;
   const uint32_t c_far = c_visit - c_exact - uint32_t(it);
-  if (COUNT && lane == 0) {
+  if (count && lane == 0) {
     atomicAdd(&st->wn_visits, (unsigned long long)c_visit);
     atomicAdd(&st->wn_far, (unsigned long long)c_far);
     atomicAdd(&st->wn_exact, (unsigned long long)c_exact);
@@ -1474,18 +1475,19 @@ __device__ __forceinline__ float wn_traverse(F3 q, const float4* __restrict__ in
 
 // Band voxel act[i] of the warp: its grid point and, after the traversal, the
 // sign of its distance (mesh_to_volume.rs:264-271).
-template <int ORDER, bool COUNT = true>
+template <int ORDER>
 __device__ __forceinline__ void wn_warp(const uint32_t* __restrict__ act, uint64_t i, bool valid, uint64_t last,
                                         const int4* __restrict__ origins, float* __restrict__ values,
                                         const float4* __restrict__ inode, const float4* __restrict__ leaf,
                                         const float4* __restrict__ inode3, const float4* __restrict__ leaf3, int n,
-                                        float h, float beta, float thresh, M2VStats* st, int (*stk)[WN_STACK]) {
+                                        float h, float beta, float thresh, M2VStats* st, int (*stk)[WN_STACK],
+                                        bool count = true) {
   const uint32_t v = valid ? act[i] : act[last];
   const uint32_t b = v >> 9, o = v & 511;
   const int4 org = origins[b];
   const F3 q = f3(fmul(__int2float_rn(org.x + int(o >> 6)), h), fmul(__int2float_rn(org.y + int((o >> 3) & 7)), h),
                   fmul(__int2float_rn(org.z + int(o & 7)), h));
-  const float sum = wn_traverse<ORDER, COUNT>(q, inode, leaf, inode3, leaf3, n, beta, st, stk);
+  const float sum = wn_traverse<ORDER>(q, inode, leaf, inode3, leaf3, n, beta, st, stk, count);
   if (valid) {
     const float d = values[uint64_t(b) * 512 + o];
     values[uint64_t(b) * 512 + o] = (sum < thresh) ? copysignf(d, 1.0f) : copysignf(d, -1.0f);
@@ -1538,9 +1540,9 @@ __global__ void __launch_bounds__(WN_THREADS) k_wn_sign_batch(const uint32_t* __
                int(M.n_tri), M.h, M.beta, M.thresh, stats + mesh, stk);
 }
 
-// The warps that the filter (fast_sign.cu) did not settle: rest[0 .. *n_rest),
-// each by its first index into act.  They are few (0.2 % of a scan's) and
-// counted there.
+// The warps that the filter (fast_sign.cu) did not settle, each by its first
+// index into act: n_rest[0] from rest[0] up, whose work is counted there, and
+// n_rest[1] from rest[n_warps - 1] down, counted here.
 __global__ void __launch_bounds__(WN_THREADS) k_wn_sign_rest(const uint32_t* __restrict__ act,
                                                              const uint32_t* __restrict__ act_base, int K,
                                                              const MeshInfo* __restrict__ mi,
@@ -1550,19 +1552,19 @@ __global__ void __launch_bounds__(WN_THREADS) k_wn_sign_rest(const uint32_t* __r
                                                              float* __restrict__ values,
                                                              const float4* __restrict__ inodes,
                                                              const float4* __restrict__ leaves, M2VStats* stats,
-                                                             const uint32_t* __restrict__ rest,
+                                                             const uint32_t* __restrict__ rest, uint32_t n_warps,
                                                              const uint32_t* __restrict__ n_rest) {
   __shared__ int stk[WN_WARPS][WN_STACK];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const uint32_t n = *n_rest;
+  const uint32_t n0 = n_rest[0], n = n0 + n_rest[1];
   for (uint32_t r = blockIdx.x * WN_WARPS + w; r < n; r += gridDim.x * WN_WARPS) {
-    const uint64_t i0 = rest[r], i = i0 + lane;
+    const uint64_t i0 = rest[r < n0 ? r : n_warps - 1 - (r - n0)], i = i0 + lane;
     const int mesh = find_seg(act_base, K, i0);
     const uint64_t a1 = act_base[mesh + 1];
     const MeshInfo M = mi[mesh];
-    wn_warp<2, false>(act, i, i < a1, a1 - 1, origins, values, inodes + 5 * uint64_t(inode_base[mesh]),
-                      leaves + 5 * uint64_t(tri_base[mesh]), nullptr, nullptr, int(M.n_tri), M.h, M.beta, M.thresh,
-                      stats + mesh, stk);
+    wn_warp<2>(act, i, i < a1, a1 - 1, origins, values, inodes + 5 * uint64_t(inode_base[mesh]),
+               leaves + 5 * uint64_t(tri_base[mesh]), nullptr, nullptr, int(M.n_tri), M.h, M.beta, M.thresh,
+               stats + mesh, stk, r >= n0);
   }
 }
 
@@ -2231,16 +2233,18 @@ static std::vector<bs_volume*> batch_core(bs_ctx* ctx, const float* d_xyz, const
                                   mi[0].h, mi[0].beta, mi[0].thresh, st.p)))
     const int ww = ctx->tune_wn_warps;
     if (!any3) {
-      DBuf<uint32_t> rest(ctx, n_warps + 1);  // listed warps, and their number
-      BS_CUDA(cudaMemsetAsync(rest.p + n_warps, 0, sizeof(uint32_t), s));
+      DBuf<uint32_t> rest(ctx, n_warps + 2);  // listed warps, and their two numbers
+      BS_CUDA(cudaMemsetAsync(rest.p + n_warps, 0, 2 * sizeof(uint32_t), s));
       static_assert(offsetof(M2VStats, wn_exact) == offsetof(M2VStats, wn_visits) + 16 && sizeof(M2VStats) % 8 == 0,
                     "the filter adds to three consecutive counters");
       fast_sign(ctx, act.p, act_base.p, d_wb.p + K + 1, span_base[K], K, d_fm.p, origins.p, values.p, frec.p,
-                nt - uint64_t(K), inode.p, leaf.p, rest.p, rest.p + n_warps, &st.p->wn_visits,
+                nt - uint64_t(K), inode.p, leaf.p, rest.p, uint32_t(n_warps), rest.p + n_warps, &st.p->wn_visits,
                 uint32_t(sizeof(M2VStats) / 8));
-      const unsigned grid = unsigned(std::min<uint64_t>(blocks(n_warps, WN_WARPS), uint64_t(8 * 152)));
+      int n_sm = 0;
+      BS_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, ctx->device));
+      const unsigned grid = unsigned(std::min<uint64_t>(blocks(n_warps, WN_WARPS), uint64_t(n_sm) * 8));
       BS_KERNEL(ctx, "k_wn_sign_rest", (k_wn_sign_rest<<<grid, WN_THREADS, 0, s>>>(act.p, act_base.p, K, d_mi.p, d_tb.p, d_ib.p, origins.p,
-                                                                               values.p, inode.p, leaf.p, st.p, rest.p, rest.p + n_warps)));
+                                                                               values.p, inode.p, leaf.p, st.p, rest.p, uint32_t(n_warps), rest.p + n_warps)));
     } else if (K == 1) {
       if (ww == 2)
         BS_WN3(2);

@@ -1,0 +1,49 @@
+"""The work counters of a conversion's sign pass (bs_ctx_last_counters [10],
+[11], and on the library's tree [6]) count every voxel's cut once, whoever
+walks it: the certified filter, or the traversal where the filter has no room
+for the cut or is not used.  They equal the counters of WindingNumbers on the
+same tree at the same points (on the library's tree in the pass's order, 32
+points per cut)."""
+import numpy as np
+import pytest
+
+import baby_shark_gb300 as bs
+from baby_shark_gb300 import synthetic
+from tests.gpu_common import context, unpack_mask
+from tests.test_gpu_fast_sign import MORTON
+from tests.test_gpu_fast_sign import convert as convert_fast
+from tests.test_gpu_sign_filter import convert as convert_reference
+from tests.test_gpu_sign_filter import shapes
+
+pytestmark = pytest.mark.gpu
+KEYS = {"fast": ("wn_warp_visits", "wn_far", "wn_exact"), "reference": ("wn_far", "wn_exact")}
+
+
+def cases():
+    s = shapes()
+    out = {k: (*s[k], 2.0) for k in ("torus", "on_grid", "degenerate", "tiny", "out_of_range", "coarse", "few2")}
+    # every node near: the pending nodes of 32 voxels outgrow the filter's stacks
+    out["all_near"] = (*synthetic.torus(1.0, 0.3, 400, 200, 0.02, seed=3), 0.2, 1, 500.0)
+    return out
+
+
+@pytest.mark.parametrize("tree", ["fast"])
+@pytest.mark.parametrize("name", sorted(cases()))
+def test_counters_equal_the_traversal(name, tree):
+    v, f, h, band, beta = cases()[name]
+    vol = convert_fast([(v, f)], [(h, band)], beta, 0.2)[0] if tree == "fast" else \
+        convert_reference(v, f, h, band, beta, 0.2)
+    st = context().last_stats()
+    o, _, m = vol.export()
+    li, k = np.nonzero(np.stack([unpack_mask(x) for x in m])[:, MORTON])
+    vi = MORTON[k]
+    pts = (o[li] + np.stack([vi >> 6, (vi >> 3) & 7, vi & 7], 1)).astype(np.float32) * np.float32(h)
+    wn = bs.WindingNumbers.from_mesh((v, f), ctx=context(), tree=tree)
+    want = dict.fromkeys(KEYS[tree], 0)
+    for i in range(0, len(pts), 1 << 19):  # larger sets are reordered
+        wn.approximate(pts[i:i + (1 << 19)], beta)
+        got = context().last_stats()
+        for key in want:
+            want[key] += got[key]
+    assert len(pts) > 0 and want["wn_far"] + want["wn_exact"] > 0
+    assert {key: st[key] for key in want} == want
