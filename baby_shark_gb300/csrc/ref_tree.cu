@@ -49,7 +49,7 @@ namespace {
 
 constexpr int NB = 12;                 // buckets per axis (aabb_tree.rs:437)
 constexpr uint32_t MIN_LEAF = 3;       // with_min_objects_per_leaf(3) (aabb_tree.rs:640)
-constexpr int MAX_DEPTH = 40;          // AABBTree's default max depth (aabb_tree.rs:69)
+constexpr int MAX_DEPTH = RT_MAX_DEPTH;
 constexpr uint32_t SMALL = 512;        // nodes up to this many triangles are finished by one CTA
 // Positions per block in the passes over large nodes.  Few, so that the passes
 // fill the SMs: k_rt_place took 0.214 ms for the nine levels of 81,920 triangles

@@ -44,6 +44,8 @@ void build_ref_trees(bs_ctx* ctx, const float4* T, uint64_t nt, int K, const uin
 void ref_tree_set_beta(bs_ctx* ctx, RefTrees& t, const std::vector<float>& beta);
 
 // Per-mesh parameters of the sign pass over band voxels.
+constexpr int RT_MAX_DEPTH = 40;  // AABBTree's default max depth (aabb_tree.rs:69); the root's is 1
+
 struct RefSignMesh {
   int root;
   float h, beta, thresh;

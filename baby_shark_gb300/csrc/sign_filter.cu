@@ -279,7 +279,10 @@ __global__ void __launch_bounds__(32 * WARPS) k_rt_sign(
         pos = n_front;
       }
       while (sp > 0 || pos < n_front) {
-        const int n1 = min(sp, 32), n2 = min(32 - n1, n_front - pos), n = n1 + n2;
+        // fewer where the stack fills: with RT_MAX_DEPTH left it goes one node
+        // at a time, deepest first, and needs one more entry per level
+        const int most = min(32, max(1, GSTACK - RT_MAX_DEPTH - sp));
+        const int n1 = min(sp, most), n2 = min(most - n1, n_front - pos), n = n1 + n2;
         const bool have = lane < n;
         int2 it = make_int2(0, 0);
         if (lane < n1) it = stk[sp - n1 + lane];
@@ -375,7 +378,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_rt_sign(
         }
         const bool open = near && ref >= 0;
         const unsigned m_o = __ballot_sync(FULLM, open);
-        if (sp + 2 * __popc(m_o) > GSTACK) {
+        if (sp + 2 * __popc(m_o) > GSTACK) {  // only in a tree deeper than RT_MAX_DEPTH
           over = true;
           break;
         }

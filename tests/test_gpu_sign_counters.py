@@ -27,7 +27,7 @@ def cases():
     return out
 
 
-@pytest.mark.parametrize("tree", ["fast"])
+@pytest.mark.parametrize("tree", ["reference", "fast"])
 @pytest.mark.parametrize("name", sorted(cases()))
 def test_counters_equal_the_traversal(name, tree):
     v, f, h, band, beta = cases()[name]
