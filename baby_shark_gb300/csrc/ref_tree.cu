@@ -1102,10 +1102,14 @@ __device__ __forceinline__ void flush_counts(const Counts& c, unsigned long long
 constexpr int SIGN_WARPS = REF_SIGN_WARPS;
 
 // The band voxels the filter left undecided (mesh_to_volume.rs:245-280): a
-// warp takes a few of one mesh at a time; the lists' lengths are on the
-// device, so a grid of resident blocks walks them.
+// warp takes a few of one list at a time; the lists' lengths are on the
+// device, so a grid of resident blocks walks them.  Mesh m's two lists lie
+// between act_base[m] + 32 leaf_base[m] and the next mesh's: list 2 m, voxels
+// whose work the filter counted, from its start up, and list 2 m + 1, whose it
+// did not, from its end down, in blocks of 32 with NO_VOXEL past a brick's last.
 __global__ void __launch_bounds__(32 * SIGN_WARPS) k_rt_sign_exact(const uint32_t* __restrict__ list,
-                                                                   const uint32_t* __restrict__ list_base,
+                                                                   const uint32_t* __restrict__ act_base,
+                                                                   const uint32_t* __restrict__ leaf_base,
                                                                    const uint32_t* __restrict__ count,
                                                                    const uint32_t* __restrict__ warp_base, int K,
                                                                    const RefSignMesh* __restrict__ meshes,
@@ -1119,24 +1123,30 @@ __global__ void __launch_bounds__(32 * SIGN_WARPS) k_rt_sign_exact(const uint32_
                                                                    unsigned long long* __restrict__ counters) {
   __shared__ WarpStack ws[SIGN_WARPS];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const uint32_t n_warps = warp_base[K], per = warp_base[K + 1];
+  const uint32_t n_warps = warp_base[2 * K], per = warp_base[2 * K + 1];
   for (uint64_t gw = blockIdx.x * uint64_t(SIGN_WARPS) + w; gw < n_warps; gw += uint64_t(gridDim.x) * SIGN_WARPS) {
-    const int m = K > 1 ? mesh_of(warp_base, K, gw) : 0;
-    const uint32_t i = uint32_t(gw - warp_base[m]) * per + lane, n = count[m];
-    const bool ok = uint32_t(lane) < per && i < n;
+    const int l = mesh_of(warp_base, 2 * K, gw), m = l >> 1;
+    const uint32_t i = uint32_t(gw - warp_base[l]) * per + lane, n = count[l];
+    const uint64_t first = (l & 1) ? act_base[m + 1] + 32 * uint64_t(leaf_base[m + 1]) - n
+                                   : act_base[m] + 32 * uint64_t(leaf_base[m]);
+    const uint32_t mine = uint32_t(lane) < per && i < n ? list[first + i] : NO_VOXEL;
+    const bool ok = mine != NO_VOXEL;
+    const unsigned valid = __ballot_sync(FULL, ok);
+    if (!valid) continue;  // the end of a block
     const RefSignMesh M = meshes[m];
-    const uint32_t v = list[uint64_t(list_base[m]) + (ok ? i : n - 1)];
+    const uint32_t other = __shfl_sync(FULL, mine, __ffs(valid) - 1), v = ok ? mine : other;
     const uint32_t b = v >> 9, o = v & 511;
     const int4 org = origins[b];
     const F3 q = f3(fmul(__int2float_rn(org.x + int(o >> 6)), M.h), fmul(__int2float_rn(org.y + int((o >> 3) & 7)), M.h),
                     fmul(__int2float_rn(org.z + int(o & 7)), M.h));
     Counts c;
-    const float wn = ref_wn_warp(q, __ballot_sync(FULL, ok), M.root, rec_i, opn, rec_l, leaf_cnt, tri, ws[w], c);
+    const float wn = ref_wn_warp(q, valid, M.root, rec_i, opn, rec_l, leaf_cnt, tri, ws[w], c);
     if (ok) {
       const float d = values[uint64_t(b) * 512 + o];
       values[uint64_t(b) * 512 + o] = (wn < M.thresh) ? copysignf(d, 1.0f) : copysignf(d, -1.0f);
     }
-    if (lane == 0 && c.overflow) atomicAdd(counters + 3, 1ull);
+    if (l & 1) flush_counts(c, counters);
+    else if (lane == 0 && c.overflow) atomicAdd(counters + 3, 1ull);
     __syncwarp();
   }
 }
@@ -1292,15 +1302,15 @@ void ref_tree_set_beta(bs_ctx* ctx, RefTrees& t, const std::vector<float>& beta)
 unsigned ref_tree_sign_exact_grid(bs_ctx* ctx, uint64_t max_list) {
   int n_sm = 0;
   BS_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, ctx->device));
-  return unsigned(std::min<uint64_t>(nblk(max_list, SIGN_WARPS), uint64_t(n_sm) * 8));
+  return unsigned(std::min<uint64_t>(nblk(max_list, SIGN_WARPS), uint64_t(n_sm) * 16));
 }
 
 void ref_tree_sign_exact(bs_ctx* ctx, const RefTrees& t, unsigned grid, const uint32_t* list,
-                         const uint32_t* d_list_base, const uint32_t* d_count, const uint32_t* d_warps, int K,
-                         const RefSignMesh* d_meshes, const int4* origins, float* values,
+                         const uint32_t* d_act_base, const uint32_t* d_leaf_base, const uint32_t* d_count,
+                         const uint32_t* d_warps, int K, const RefSignMesh* d_meshes, const int4* origins, float* values,
                          unsigned long long* d_counters) {
   BS_KERNEL(ctx, "k_rt_sign_exact", (k_rt_sign_exact<<<grid, 32 * SIGN_WARPS, 0, ctx->stream>>>(
-                                        list, d_list_base, d_count, d_warps, K, d_meshes, origins, values, t.rec_i.p,
+                                        list, d_act_base, d_leaf_base, d_count, d_warps, K, d_meshes, origins, values, t.rec_i.p,
                                         t.open.p, t.rec_l.p, t.leaf_cnt.p, t.tri.p, d_counters)));
 }
 

@@ -106,6 +106,16 @@ struct SignSmem {
   unsigned long long cnt[6];
 };
 
+// All of a brick's voxels to the traversal, in warps of their own: `end` is where its mesh's room ends.
+__device__ __noinline__ void hand_over(const uint32_t* __restrict__ act, uint32_t nv, uint64_t end, uint32_t* n_uncounted,
+                                       uint32_t* __restrict__ undecided, uint32_t* at) {
+  const uint32_t n = (nv + 31u) & ~31u;
+  if (threadIdx.x == 0) *at = atomicAdd(n_uncounted, n);
+  __syncthreads();
+  end -= *at + uint64_t(n);
+  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) undecided[end + i] = i < nv ? act[i] : NO_VOXEL;
+}
+
 // One CTA per brick: its first warp runs the brick's phase, then every warp
 // takes the next 32 voxels.  Issue-bound (like the exact traversal): 62.6 ms
 // with the exact traversal of every voxel, 15.1 ms here, on a torus of 1 M
@@ -153,12 +163,16 @@ __global__ void __launch_bounds__(32 * WARPS) k_rt_sign(
   }
   __syncthreads();
   // Distances from any voxel to any vertex or dipole centre of the mesh stay
-  // below R2_MAX when the root's sphere and this brick do.
+  // below R2_MAX (past which the bound does not hold) when the root's sphere and this brick do.
   WorkCounts wc;
   float4 Hroot = frec[4 * uint64_t(rec_index(M.root, nt))];
   const float root_r = M.root >= 0 ? rad_i[M.root] : rad_l[~M.root];
   const float reach = root_r + (fabsf(Hroot.x - bcx) + fabsf(Hroot.y - bcy) + fabsf(Hroot.z - bcz)) + 16.0f * M.h;
-  const bool in_range = reach * reach < R2_MAX;  // false for NaN
+  if (!(reach * reach < R2_MAX)) {  // NaN too
+    hand_over(act + v0, nv, uint64_t(act_base[mesh + 1]) + 32 * uint64_t(leaf_base[mesh + 1]),
+              n_undecided + 2 * mesh + 1, undecided, &sm.rho2);
+    return;
+  }
 
   // ---- brick phase: warp 0 ----
   if (w == 0) {
@@ -268,7 +282,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_rt_sign(
       taylor_clear(T);
       Lane s;
       s.w = s.mag = s.etri = 0.0f;
-      s.bad = !in_range;
+      s.bad = false;
       uint32_t n_add = 0;
       bool over = false;
       int sp = 0, pos = 0;
@@ -430,9 +444,10 @@ __global__ void __launch_bounds__(32 * WARPS) k_rt_sign(
     }
     if (lanes) {
       uint32_t base = 0;
-      if (lane == 0) base = atomicAdd(n_undecided + mesh, uint32_t(__popc(lanes)));
+      if (lane == 0) base = atomicAdd(n_undecided + 2 * mesh, uint32_t(__popc(lanes)));
       base = __shfl_sync(FULLM, base, 0);
-      if ((lanes >> lane) & 1u) undecided[act_base[mesh] + base + __popc(lanes & lt)] = vox;
+      if ((lanes >> lane) & 1u)
+        undecided[uint64_t(act_base[mesh]) + 32 * uint64_t(leaf_base[mesh]) + base + __popc(lanes & lt)] = vox;
     }
     __syncwarp();
   }
@@ -451,25 +466,34 @@ __global__ void __launch_bounds__(32 * WARPS) k_rt_sign(
   if (threadIdx.x < 6 && sm.cnt[threadIdx.x]) atomicAdd(counters + threadIdx.x, sm.cnt[threadIdx.x]);
 }
 
-// Work split of the exact pass: base[m] = first warp of mesh m, base[K + 1] =
-// voxels per warp.  A warp walks the union of its voxels' cuts, and the few
-// undecided voxels are scattered over the mesh, so as long as warps are free a
-// warp takes fewer voxels (one, when n_warps suffice for all).
-__global__ void k_undecided_warps(const uint32_t* __restrict__ n_undecided, int K, uint32_t n_warps,
+// Work split of the exact pass over n lists: base[l] = first warp of list l,
+// base[n + 1] = voxels per warp.  A warp walks the union of its voxels' cuts,
+// and the few undecided voxels are scattered over the mesh, so as long as warps
+// are free a warp takes fewer voxels (one, when n_warps suffice for all).  A
+// power of two, which keeps 32 voxels that were listed together together.
+__global__ void k_undecided_warps(const uint32_t* __restrict__ n_undecided, int n, uint32_t n_warps,
                                   uint32_t* __restrict__ base) {
   const int lane = threadIdx.x;
   unsigned long long total = 0;
-  for (int m = lane; m < K; m += 32) total += n_undecided[m];
+  for (int l = lane; l < n; l += 32) total += n_undecided[l];
   for (int d = 16; d > 0; d >>= 1) total += __shfl_xor_sync(FULLM, total, d);
-  const uint32_t per = uint32_t(min((unsigned long long)32, max(1ull, (total + n_warps - 1) / n_warps)));
-  if (lane) return;
+  uint32_t per = 1;
+  while (per < 32 && uint64_t(per) * n_warps < total) per *= 2;
   uint32_t at = 0;
-  for (int m = 0; m < K; ++m) {
-    base[m] = at;
-    at += (n_undecided[m] + per - 1) / per;
+  for (int l0 = 0; l0 < n; l0 += 32) {
+    const uint32_t mine = l0 + lane < n ? (n_undecided[l0 + lane] + per - 1) / per : 0u;
+    uint32_t end = mine;
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t v = __shfl_up_sync(FULLM, end, d);
+      if (lane >= d) end += v;
+    }
+    if (l0 + lane < n) base[l0 + lane] = at + end - mine;
+    at += __shfl_sync(FULLM, end, 31);
   }
-  base[K] = at;
-  base[K + 1] = per;
+  if (lane == 0) {
+    base[n] = at;
+    base[n + 1] = per;
+  }
 }
 
 }  // namespace
@@ -479,9 +503,9 @@ void ref_tree_sign(bs_ctx* ctx, const RefTrees& t, const uint32_t* act, const ui
                    const RefSignMesh* d_meshes, const int4* origins, float* values, unsigned long long* d_counters) {
   if (n_act == 0) return;
   cudaStream_t s = ctx->stream;
-  DBuf<uint32_t> und(ctx, n_act), n_und(ctx, K), warps(ctx, K + 2);
+  DBuf<uint32_t> und(ctx, n_act + 32 * n_bricks), n_und(ctx, 2 * K), warps(ctx, 2 * K + 2);
   DBuf<float4> frec(ctx, 8 * t.nt);
-  BS_CUDA(cudaMemsetAsync(n_und.p, 0, K * sizeof(uint32_t), s));
+  BS_CUDA(cudaMemsetAsync(n_und.p, 0, 2 * K * sizeof(uint32_t), s));
   BS_KERNEL(ctx, "k_rt_filter_records", (k_rt_filter_records<<<unsigned((t.nt + 255) / 256), 256, 0, s>>>(
                                             t.nt, t.flags.p, t.topo.p, t.leaf_cnt.p, t.rec_i.p, t.rec_l.p, frec.p)));
 #define BS_RT_SIGN(W)                                                                                                  \
@@ -496,9 +520,13 @@ void ref_tree_sign(bs_ctx* ctx, const RefTrees& t, const uint32_t* act, const ui
     BS_RT_SIGN(4);
 #undef BS_RT_SIGN
   const unsigned grid = ref_tree_sign_exact_grid(ctx, n_act);
+  int n_sm = 0;
+  BS_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, ctx->device));
+  const uint32_t enough = std::min(grid * REF_SIGN_WARPS, unsigned(n_sm) * 32);
   BS_KERNEL(ctx, "k_undecided_warps",
-            (k_undecided_warps<<<1, 32, 0, s>>>(n_und.p, K, grid * REF_SIGN_WARPS, warps.p)));
-  ref_tree_sign_exact(ctx, t, grid, und.p, d_act_base, n_und.p, warps.p, K, d_meshes, origins, values, d_counters);
+            (k_undecided_warps<<<1, 32, 0, s>>>(n_und.p, 2 * K, enough, warps.p)));
+  ref_tree_sign_exact(ctx, t, grid, und.p, d_act_base, d_leaf_base, n_und.p, warps.p, K, d_meshes, origins, values,
+                      d_counters);
 }
 
 }  // namespace bs

@@ -1,0 +1,58 @@
+"""What the sign pass of a conversion costs where its certified filter settles
+little or nothing, against the traversal of the same points (WindingNumbers on
+the same tree; device times of the kernels, best of four): the filter must
+not cost more than it saves.  Where it works it takes a third to a half of the
+traversal's time; the bound leaves room for the events around short kernels."""
+import numpy as np
+import pytest
+
+import baby_shark_gb300 as bs
+from baby_shark_gb300 import synthetic
+from tests.gpu_common import context, unpack_mask
+from tests.test_gpu_fast_sign import MORTON
+from tests.test_gpu_fast_sign import convert as convert_fast
+from tests.test_gpu_sign_filter import convert as convert_reference
+
+pytestmark = pytest.mark.gpu
+MOST = 1.3
+
+
+def cases():
+    v, f = synthetic.torus(1.0, 0.3, 256, 128, 0.02, seed=3)
+    return {"out_of_range": (v * np.float32(2e6), f, 0.012 * 2e6, 2, 2.0)}
+
+
+def stages(run, names):
+    """Best device time of the named kernels together, in ms."""
+    ctx, best = context(), 1e9
+    ctx.set_stage_timing(True)
+    try:
+        for _ in range(4):
+            ctx.stage_times(reset=True)
+            out = run()
+            t = ctx.stage_times(reset=True)
+            best = min(best, sum(ms for k, (ms, _) in t.items() if k in names))
+    finally:
+        ctx.set_stage_timing(False)
+    return out, best
+
+
+@pytest.mark.parametrize("tree,name", [("reference", "out_of_range")])
+def test_sign_pass_against_the_traversal(tree, name):
+    v, f, h, band, beta = cases()[name]
+
+    def convert():
+        if tree == "fast":
+            return convert_fast([(v, f)], [(h, band)], beta, 0.2)[0]
+        return convert_reference(v, f, h, band, beta, 0.2)
+
+    vol, mine = stages(convert, ("k_rt_sign", "k_undecided_warps", "k_rt_sign_exact", "k_wn_sign", "k_wn_sign_rest"))
+    o, _, m = vol.export()
+    li, k = np.nonzero(np.stack([unpack_mask(x) for x in m])[:, MORTON])
+    vi = MORTON[k]
+    pts = (o[li] + np.stack([vi >> 6, (vi >> 3) & 7, vi & 7], 1)).astype(np.float32) * np.float32(h)
+    assert 0 < len(pts) < 1 << 20  # larger sets are reordered
+    wn = bs.WindingNumbers.from_mesh((v, f), ctx=context(), tree=tree)
+    _, theirs = stages(lambda: wn.approximate(pts, beta), ("k_rt_points", "k_wn_points"))
+    print("%s %s: sign pass %.3f ms, traversal %.3f ms" % (tree, name, mine, theirs))
+    assert 0 < mine <= MOST * theirs
