@@ -11,8 +11,8 @@
 // the traversal's.
 //
 // What makes it cheap: nodes are tested 32 at a time, one per lane, against
-// the bounding sphere and box of the voxels (of FAST_SIGN_SPAN consecutive
-// ones first, then of each 32), and where these leave a node open its lane
+// the bounding sphere and box of the voxels (of up to 256 consecutive ones
+// first, then of each 32), and where these leave a node open its lane
 // goes through the voxels; far nodes with a small enough truncation error
 // enter one Taylor polynomial, lane by lane; only close far nodes and the near
 // triangles are evaluated by every voxel.
@@ -92,7 +92,7 @@ struct FastSmem {  // of a warp
   float taylor[11];  // the span's polynomial
 };
 
-// Every warp takes FAST_SIGN_SPAN voxels by itself.  Issue-bound: about 16 k
+// Every warp takes a span of voxels by itself.  Issue-bound: about 16 k
 // instructions per 32 voxels, of which the far fields per voxel (125 nodes)
 // take a quarter and the tests, the polynomials and the triangles (17) a fifth
 // each.  On a scan of 1.2 M triangles with holes and 14.7 M band voxels: 13.8
@@ -102,11 +102,13 @@ struct FastSmem {  // of a warp
 // 32 warps per SM with spills: +0.1, +0.2 ms; testing a node with a vote of
 // all voxels instead of in a loop over them on its lane: +0.6 ms; E_GROUP
 // 0.045: +0.3 ms (5 % of the groups take the second attempt).
+constexpr int WARPS_PER_SM = 24, SPAN_WAVES = 4;
+
 template <int WARPS>
-__global__ void __launch_bounds__(32 * WARPS, 24 / WARPS) k_wn_filter(
+__global__ void __launch_bounds__(32 * WARPS, WARPS_PER_SM / WARPS) k_wn_filter(
     const uint32_t* __restrict__ act, const uint32_t* __restrict__ act_base, const uint32_t* __restrict__ span_base,
-    int K, const FastSignMesh* __restrict__ meshes, const int4* __restrict__ origins, float* __restrict__ values,
-    const float4* __restrict__ frec0, uint64_t ni, const float4* __restrict__ inode, const float4* __restrict__ leaf0,
+    uint32_t span_size, int K, const FastSignMesh* __restrict__ meshes, const int4* __restrict__ origins,
+    float* __restrict__ values, const float4* __restrict__ frec0, uint64_t ni, const float4* __restrict__ inode, const float4* __restrict__ leaf0,
     uint32_t* __restrict__ rest, uint32_t n_warps, uint32_t* __restrict__ n_rest,
     unsigned long long* __restrict__ counts, uint32_t count_stride) {
   __shared__ FastSmem smem[WARPS];
@@ -117,8 +119,8 @@ __global__ void __launch_bounds__(32 * WARPS, 24 / WARPS) k_wn_filter(
   FastSmem& sm = smem[threadIdx.x >> 5];
   const int mesh = K > 1 ? segment(span_base, K, span) : 0;
   const FastSignMesh M = meshes[mesh];
-  const uint32_t i0 = act_base[mesh] + (span - span_base[mesh]) * uint32_t(FAST_SIGN_SPAN);
-  const uint32_t nv = min(uint32_t(FAST_SIGN_SPAN), act_base[mesh + 1] - i0);
+  const uint32_t i0 = act_base[mesh] + (span - span_base[mesh]) * span_size;
+  const uint32_t nv = min(span_size, act_base[mesh + 1] - i0);
   const float4* frec_i = frec0 + 4 * uint64_t(M.inode_base);
   const float4* frec_l = frec0 + 4 * (ni + M.tri_base);
   const float4* leaf = leaf0 + 5 * uint64_t(M.tri_base);
@@ -417,14 +419,26 @@ void fast_filter_records(bs_ctx* ctx, const float4* inode, uint64_t n_internal, 
                 inode, n_internal, d_inode_base, leaf, nt, d_tri_base, K, d_meshes, frec)));
 }
 
+// Consecutive active voxels of a mesh that one warp takes, for n_act of them in
+// all: 32, 64, 128 or 256.  The longer a span, the more its groups share; but
+// a warp takes its groups one after another, so the spans must fill the SMs
+// several times over.
+uint32_t fast_sign_span(bs_ctx* ctx, uint64_t n_act) {
+  int n_sm = 0;
+  BS_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, ctx->device));
+  uint32_t span = 256;
+  while (span > 32 && n_act < uint64_t(span) * SPAN_WAVES * WARPS_PER_SM * unsigned(n_sm)) span /= 2;
+  return span;
+}
+
 void fast_sign(bs_ctx* ctx, const uint32_t* act, const uint32_t* d_act_base, const uint32_t* d_span_base,
-               uint32_t n_spans, int K, const FastSignMesh* d_meshes, const int4* origins, float* values,
+               uint32_t span, uint32_t n_spans, int K, const FastSignMesh* d_meshes, const int4* origins, float* values,
                const float4* frec, uint64_t n_internal, const float4* inode, const float4* leaf, uint32_t* rest,
                uint32_t n_warps, uint32_t* n_rest, unsigned long long* d_counts, uint32_t count_stride) {
   if (n_spans == 0) return;
 #define BS_WN_FILTER(W)                                                                                            \
   BS_KERNEL(ctx, "k_wn_sign", (k_wn_filter<W><<<(n_spans + W - 1) / W, 32 * W, 0, ctx->stream>>>(                                \
-                                  act, d_act_base, d_span_base, K, d_meshes, origins, values, frec, n_internal,    \
+                                  act, d_act_base, d_span_base, span, K, d_meshes, origins, values, frec, n_internal,    \
                                   inode, leaf, rest, n_warps, n_rest, d_counts, count_stride)))
   if (ctx->tune_wn_warps == 2)
     BS_WN_FILTER(2);

@@ -22,18 +22,19 @@ __device__ __forceinline__ float cut_dist2(float rx, float ry, float rz) {
   return __fmaf_rn(rz, rz, __fmaf_rn(rx, rx, __fmul_rn(ry, ry)));
 }
 
-// Consecutive active voxels of a mesh that one warp takes.
-constexpr int FAST_SIGN_SPAN = 256;
+// Consecutive active voxels of a mesh that one warp takes, for n_act of them
+// in all.
+uint32_t fast_sign_span(bs_ctx* ctx, uint64_t n_act);
 
 // Signs the active voxels of K meshes as wn_warp would (m2v.cu), except those
 // of the warps it lists (by their first index into act) in rest: n_rest[0] of
 // them from rest[0] up, n_rest[1] from rest[n_warps - 1] down.  span_base[m] ..
-// span_base[m + 1] are mesh m's spans of FAST_SIGN_SPAN voxels of
+// span_base[m + 1] are mesh m's spans of `span` voxels of
 // act[act_base[m], act_base[m + 1]).  Mesh m's node visits, far fields and
 // solid angles of the warps' cuts are added to counts[m * count_stride] and
 // the two after it, those of the n_rest[1] warps left to their traversal.
 void fast_sign(bs_ctx* ctx, const uint32_t* act, const uint32_t* d_act_base, const uint32_t* d_span_base,
-               uint32_t n_spans, int K, const FastSignMesh* d_meshes, const int4* origins, float* values,
+               uint32_t span, uint32_t n_spans, int K, const FastSignMesh* d_meshes, const int4* origins, float* values,
                const float4* frec, uint64_t n_internal, const float4* inode, const float4* leaf, uint32_t* rest,
                uint32_t n_warps, uint32_t* n_rest, unsigned long long* d_counts, uint32_t count_stride);
 

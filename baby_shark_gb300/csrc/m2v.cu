@@ -2200,10 +2200,11 @@ static std::vector<bs_volume*> batch_core(bs_ctx* ctx, const float* d_xyz, const
   // per mesh its first warp, then its first span of the filter pass
   std::vector<uint32_t> warp_base(2 * (K + 1), 0);
   uint32_t* span_base = warp_base.data() + K + 1;
+  const uint32_t span = fast_sign_span(ctx, na);
   for (int m = 0; m < K; ++m) {
     const uint32_t n_act = h_act_base[m + 1] - h_act_base[m];
     warp_base[m + 1] = warp_base[m] + (n_act + 31) / 32;
-    span_base[m + 1] = span_base[m] + (n_act + FAST_SIGN_SPAN - 1) / FAST_SIGN_SPAN;
+    span_base[m + 1] = span_base[m] + (n_act + span - 1) / span;
   }
   DBuf<uint32_t> d_wb(ctx, 2 * (K + 1));
   BS_CUDA(cudaMemcpyAsync(d_wb.p, warp_base.data(), 2 * (K + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
@@ -2237,7 +2238,7 @@ static std::vector<bs_volume*> batch_core(bs_ctx* ctx, const float* d_xyz, const
       BS_CUDA(cudaMemsetAsync(rest.p + n_warps, 0, 2 * sizeof(uint32_t), s));
       static_assert(offsetof(M2VStats, wn_exact) == offsetof(M2VStats, wn_visits) + 16 && sizeof(M2VStats) % 8 == 0,
                     "the filter adds to three consecutive counters");
-      fast_sign(ctx, act.p, act_base.p, d_wb.p + K + 1, span_base[K], K, d_fm.p, origins.p, values.p, frec.p,
+      fast_sign(ctx, act.p, act_base.p, d_wb.p + K + 1, span, span_base[K], K, d_fm.p, origins.p, values.p, frec.p,
                 nt - uint64_t(K), inode.p, leaf.p, rest.p, uint32_t(n_warps), rest.p + n_warps, &st.p->wn_visits,
                 uint32_t(sizeof(M2VStats) / 8));
       int n_sm = 0;

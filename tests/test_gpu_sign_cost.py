@@ -1,8 +1,9 @@
-"""What the sign pass of a conversion costs where its certified filter settles
-little or nothing, against the traversal of the same points (WindingNumbers on
-the same tree; device times of the kernels, best of four): the filter must
-not cost more than it saves.  Where it works it takes a third to a half of the
-traversal's time; the bound leaves room for the events around short kernels."""
+"""What the sign pass of a conversion costs at the ends of its certified
+filter's range, against the traversal of the same points (WindingNumbers on
+the same tree; device times of the kernels, best of four).  Where the filter
+settles every voxel it must be the faster one (it takes a third to a half of
+the traversal's time on large meshes); where it settles nothing it must not add
+to the traversal more than the events around short kernels do."""
 import numpy as np
 import pytest
 
@@ -14,12 +15,13 @@ from tests.test_gpu_fast_sign import convert as convert_fast
 from tests.test_gpu_sign_filter import convert as convert_reference
 
 pytestmark = pytest.mark.gpu
-MOST = 1.3
+SETTLED, HANDED_OVER = 0.9, 1.3
 
 
 def cases():
     v, f = synthetic.torus(1.0, 0.3, 256, 128, 0.02, seed=3)
-    return {"out_of_range": (v * np.float32(2e6), f, 0.012 * 2e6, 2, 2.0)}
+    return {"out_of_range": (v * np.float32(2e6), f, 0.012 * 2e6, 2, 2.0),
+            "few_voxels": (*synthetic.icosphere(4, 1.0, 0.0, seed=1), 0.2, 1, 2.0)}
 
 
 def stages(run, names):
@@ -37,8 +39,8 @@ def stages(run, names):
     return out, best
 
 
-@pytest.mark.parametrize("tree,name", [("reference", "out_of_range")])
-def test_sign_pass_against_the_traversal(tree, name):
+@pytest.mark.parametrize("tree,name,most", [("reference", "out_of_range", HANDED_OVER), ("fast", "few_voxels", SETTLED)])
+def test_sign_pass_against_the_traversal(tree, name, most):
     v, f, h, band, beta = cases()[name]
 
     def convert():
@@ -55,4 +57,4 @@ def test_sign_pass_against_the_traversal(tree, name):
     wn = bs.WindingNumbers.from_mesh((v, f), ctx=context(), tree=tree)
     _, theirs = stages(lambda: wn.approximate(pts, beta), ("k_rt_points", "k_wn_points"))
     print("%s %s: sign pass %.3f ms, traversal %.3f ms" % (tree, name, mine, theirs))
-    assert 0 < mine <= MOST * theirs
+    assert 0 < mine <= most * theirs
