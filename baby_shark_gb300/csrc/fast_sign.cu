@@ -356,11 +356,15 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS_PER_SM / WARPS) k_wn_filter(
           ++n_add;
           // the traversal's own formula where it takes the unfused one for
           // certain: below its minimal length, or |num| < 1e-4 (256 u and
-          // more below that)
-          angle_add(s, A, B, C, q, [&](float an, float P, float l2) {
+          // more below that).  Else, near an edge or vertex, num and den are
+          // off by 256 u each and 0.8e-4 or more from 0 together, which moves
+          // twice the angle by at most 2 asin(sqrt(2) 256 u / max(..)) and the
+          // arctangents' errors: below 5e-5 / max(..).
+          angle_add(s, A, B, C, q, [&](float an, float P, float im, float l2, float w) {
             if (l2 < 0x1p-100f || (l2 >= 0x1p-60f && an < 0.8e-4f * P)) return exact_angle(A, B, C, q);
-            s.bad = true;
-            return 0.0f;
+            s.bad |= !(l2 >= 0x1p-60f);
+            s.etri += 5e-5f * (P * im);
+            return w;
           });
         }
         __syncwarp();

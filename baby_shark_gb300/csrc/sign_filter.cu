@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_rt_sign(
           if ((l >> lane) & 1u)
             for (uint32_t k = 0; k < c; ++k) {
               const float4 A = __ldg(tp + 3 * k), B = __ldg(tp + 3 * k + 1), C = __ldg(tp + 3 * k + 2);
-              angle_add(s, A, B, C, q, [&](float, float, float) { return exact_angle(A, B, C, q); });
+              angle_add(s, A, B, C, q, [&](float, float, float, float, float) { return exact_angle(A, B, C, q); });
             }
         }
         __syncwarp();

@@ -122,8 +122,8 @@ __device__ __forceinline__ void far_add(Lane& s, float4 A, float4 S, float na, f
 // Solid angle of a triangle at q: 2 atan2(num, den), Van Oosterom
 // and Strackee's formula on the unnormalised corner vectors.  The arctangent
 // on [0, 1] is Abramowitz and Stegun 4.4.47 (|error| <= 1e-5).  Where the
-// bound above ends (fine false; NaN too), unsettled(s, an, P, min length^2)
-// gives the value and raises the bounds.
+// bound above ends (fine false; NaN too), unsettled(an, P, 1 / max(an, |den|),
+// min length^2, this value) gives the value and raises the bounds.
 template <class Unsettled>
 __device__ __forceinline__ void angle_add(Lane& s, float4 A, float4 B, float4 C, F3 q, Unsettled unsettled) {
   const float ax = A.x - q.x, ay = A.y - q.y, az = A.z - q.z;
@@ -149,7 +149,7 @@ __device__ __forceinline__ void angle_add(Lane& s, float4 A, float4 B, float4 C,
   if (fine)
     s.etri += 1.4e-4f * (P * im);
   else
-    w = unsettled(an, P, l2);
+    w = unsettled(an, P, im, l2, w);
   s.w += w;
   s.mag += fabsf(w);
 }

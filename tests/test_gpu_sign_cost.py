@@ -21,7 +21,9 @@ SETTLED, HANDED_OVER = 0.9, 1.3
 def cases():
     v, f = synthetic.torus(1.0, 0.3, 256, 128, 0.02, seed=3)
     return {"out_of_range": (v * np.float32(2e6), f, 0.012 * 2e6, 2, 2.0),
-            "few_voxels": (*synthetic.icosphere(4, 1.0, 0.0, seed=1), 0.2, 1, 2.0)}
+            "few_voxels": (*synthetic.icosphere(4, 1.0, 0.0, seed=1), 0.2, 1, 2.0),
+            # many triangles in every voxel, some voxels near an edge or vertex of one
+            "edges": (*synthetic.torus(1.0, 0.3, 1024, 512, 0.02, seed=3), 0.02, 1, 2.0)}
 
 
 def stages(run, names):
@@ -39,7 +41,8 @@ def stages(run, names):
     return out, best
 
 
-@pytest.mark.parametrize("tree,name,most", [("reference", "out_of_range", HANDED_OVER), ("fast", "few_voxels", SETTLED)])
+@pytest.mark.parametrize("tree,name,most", [("reference", "out_of_range", HANDED_OVER), ("fast", "few_voxels", SETTLED),
+                                            ("fast", "edges", SETTLED)])
 def test_sign_pass_against_the_traversal(tree, name, most):
     v, f, h, band, beta = cases()[name]
 
