@@ -66,7 +66,8 @@ struct M2VStats {
   unsigned long long wn_far;         // warp-level far-field evaluations (internal + leaf dipoles)
   unsigned long long wn_exact;       // warp-level exact solid angles
   unsigned long long n_eval;         // (voxel, sub-triangle) pairs left after culling
-  unsigned long long area16;         // surface in sixteenths of a squared voxel (for choosing the distance pass)
+  unsigned long long area16;         // surface in sixteenths of a squared voxel and
+  unsigned long long n_uncullable;   // about how many sub-triangles are never culled (for choosing the distance pass)
 };
 
 // Per-mesh parameters of a batch.  Triangles of mesh m are [tri_base,
@@ -182,6 +183,8 @@ __device__ __forceinline__ uint64_t owner_of(const uint32_t* __restrict__ off, u
   return lo;
 }
 
+__device__ __forceinline__ void cull_coeffs(F3 ab, F3 ac, F3 cb, float R, float M, float& c2, float& E0, float& E1);
+
 // ------------------------------------------- 1. triangles and subdivision --
 __global__ void k_gather(const float* __restrict__ xyz, const uint32_t* __restrict__ tri, uint64_t nt,
                          const MeshInfo* __restrict__ mi, const uint32_t* __restrict__ tri_base, int K,
@@ -234,6 +237,18 @@ __global__ void k_gather(const float* __restrict__ xyz, const uint32_t* __restri
     const F3 n = cross3(e0, e1);
     const float a16 = 8.0f * sqrtf(dot3(n, n)) * inv_h * inv_h;
     warp_add(&S->area16, a16 < 1e9f ? uint32_t(a16) : 0u, mesh);  // 0 for NaN too
+    // whether its sub-triangles would be culled (put_subtri), their boxes' size estimated
+    const float inv_n = ns >= 2.0f ? 1.0f / ns : 1.0f;
+    const F3 s0 = scale3(e0, inv_n), s1 = scale3(e1, inv_n), s2 = scale3(e2, inv_n);
+    const F3 lo = min3(min3(s0, s1), f3(0.f, 0.f, 0.f)), hi = max3(max3(s0, s1), f3(0.f, 0.f, 0.f));
+    const float box = 2.0f * float(M.band) + 2.5f;
+    const F3 ext = f3((hi.x - lo.x) * inv_h + box, (hi.y - lo.y) * inv_h + box, (hi.z - lo.z) * inv_h + box);
+    const F3 am = max3(max3(f3(fabsf(a.x), fabsf(a.y), fabsf(a.z)), f3(fabsf(b.x), fabsf(b.y), fabsf(b.z))),
+                       f3(fabsf(c.x), fabsf(c.y), fabsf(c.z)));
+    float c2, E0, E1;
+    cull_coeffs(s0, s1, s2, h * (sqrtf(dot3(ext, ext)) + 2.0f), fmaxf(fmaxf(am.x, am.y), am.z) + float(M.band) * h, c2,
+                E0, E1);
+    if (!(c2 < INFINITY)) warp_add(&S->n_uncullable, cnt, mesh);
   }
   F3 mn = min3(c, min3(a, b)), mx = max3(c, max3(a, b));
   float lo[3] = {mn.x, mn.y, mn.z}, hi[3] = {mx.x, mx.y, mx.z};
@@ -1687,6 +1702,7 @@ bs_status exact_winding_numbers_impl(bs_ctx* ctx, const float* d_xyz, uint64_t n
 static inline unsigned blocks(uint64_t n, unsigned t) { return unsigned((n + t - 1) / t); }
 
 constexpr double PATCH_PAIRS = 130.0;  // box pairs per band voxel from which the distance pass works on patches
+constexpr uint64_t PATCH_UNCULLABLE = 16;  // sub-triangles for each that is never culled, from which it does
 
 // One set of launches for a batch of meshes (the single-mesh call is a batch
 // of one).  Every kernel covers all meshes' triangles, bricks or voxels and
@@ -2028,13 +2044,18 @@ static std::vector<bs_volume*> batch_core(bs_ctx* ctx, const float* d_xyz, const
   // Distance pass on sub-triangles / on patches at that many pairs per voxel:
   // 41: 4.2 / 5.1 ms, 88: 5.6 / 6.0, 180: 3.44 / 3.31, 192: 15.6 / 12.2,
   // 324: 12.9 / 7.8, 390: 18.9 / 11.4 (meshes of 0.8 k to 1 M triangles).
+  // Not where many sub-triangles are never culled (cull_coeffs; slender ones):
+  // every pair is evaluated then, and the pass on patches takes longer for it
+  // (20 k needles of 7.1 M sub-triangles, band 3: 25.4 / 46.4 ms).
   double est = 0.0, area = 0.0;
+  uint64_t uncullable = 0;
   for (int m = 0; m < K; ++m) {
     const double box = 2.0 * mi[m].band + 3.3;
     est += 0.61 * box * box * double(hst[m].n_sub);
     area += double(hst[m].area16) / 16.0;
+    uncullable += hst[m].n_uncullable;
   }
-  const bool patches = area > 0.0 && est > PATCH_PAIRS * area && ns >= 2 * nt;
+  const bool patches = area > 0.0 && est > PATCH_PAIRS * area && ns >= 2 * nt && PATCH_UNCULLABLE * uncullable <= ns;
   DBuf<Patch> pat;
   uint64_t n_list = ns;  // entries of the lists' kind: sub-triangles or patches
   if (patches) {

@@ -1,0 +1,54 @@
+"""Which distance pass a conversion takes (csrc/m2v.cu: on patches of
+sub-triangles where a band voxel meets many of their boxes and they can be
+culled, else on sub-triangles; the stage k_patches runs for the first alone)."""
+import numpy as np
+import pytest
+
+import baby_shark_gb300 as bs
+from baby_shark_gb300 import synthetic
+from oracle import binding as ob
+from tests.gpu_common import compare_volumes, context
+
+pytestmark = pytest.mark.gpu
+
+
+def needles(n, aspect, seed):
+    """Random triangles about 0.4 long and `aspect` of that high."""
+    rng = np.random.default_rng(seed)
+    t = rng.uniform(-0.5, 0.5, (n, 1, 3)) + 0.2 * rng.normal(size=(n, 3, 3))
+    x = t[:, 1] - t[:, 0]
+    up = np.cross(x, rng.normal(size=(n, 3)))
+    up *= (aspect * np.linalg.norm(x, axis=1) / np.linalg.norm(up, axis=1))[:, None]
+    t[:, 2] = t[:, 0] + x * rng.uniform(0.2, 0.8, (n, 1)) + up
+    v = t.astype(np.float32).reshape(-1, 3)
+    return v, np.arange(len(v), dtype=np.uint32).reshape(-1, 3)
+
+
+def convert(mesh, h, band, ctx=None):
+    """The volume, and whether the pass on patches made it."""
+    ctx = ctx or context()
+    ctx.set_stage_timing(True)
+    try:
+        ctx.stage_times(reset=True)
+        vol = bs.MeshToVolume(ctx).with_voxel_size(h).with_narrow_band_width(band).convert(mesh)
+        return vol, "k_patches" in ctx.stage_times(reset=True)
+    finally:
+        ctx.set_stage_timing(False)
+
+
+def assert_same(vol, mesh, h, band):
+    o, _, _ = ob.mesh_to_volume(*mesh, h, band)
+    rep = compare_volumes(vol.export(), o.export())
+    assert rep["leaf_set_equal"] and rep["mask_mismatch_leaves"] == 0 and rep["value_mismatch"] == 0, rep
+    assert rep["active"] > 0
+
+
+@pytest.mark.parametrize("aspect,patches", [(0.7, True), (0.003, False)])
+def test_slender_triangles_keep_the_pass_on_sub_triangles(aspect, patches):
+    """Equally many boxes per voxel; the slender triangles' sub-triangles are never culled."""
+    mesh, h, band = needles(100, aspect, 1), 0.02, 4
+    vol, took = convert(mesh, h, band)
+    assert took == patches
+    st = context().last_stats()
+    assert (st["voxel_pairs_evaluated"] < st["voxel_pairs"]) == patches
+    assert_same(vol, mesh, h, band)
