@@ -28,6 +28,10 @@ using namespace sign_filter;
 constexpr int FRONT = 448;   // nodes a warp's first phase leaves to its groups
 constexpr int STACK = 256;   // pending nodes
 constexpr float E_GROUP = 0.02f;  // truncation error of one expanded node in a group's first attempt
+// A mesh of whose groups the filter has left more than one in TALLY_SHARE (it
+// takes about 0.4 of the traversal's time, twice that with the second attempt)
+// goes to the traversal from there on, but for one span in TALLY_SAMPLE.
+constexpr uint32_t TALLY_FROM = 64, TALLY_SHARE = 3, TALLY_SAMPLE = 32;
 constexpr int SLOT = 5;      // float4 per lane's broadcast slot: 4 and one that keeps the banks apart
 // the float32 squared distances are within 4 u: outside of this the traversal's test is certain
 constexpr float TAU_LO = 0.999999f, TAU_HI = 1.000001f;
@@ -109,8 +113,8 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS_PER_SM / WARPS) k_wn_filter(
     const uint32_t* __restrict__ act, const uint32_t* __restrict__ act_base, const uint32_t* __restrict__ span_base,
     uint32_t span_size, int K, const FastSignMesh* __restrict__ meshes, const int4* __restrict__ origins,
     float* __restrict__ values, const float4* __restrict__ frec0, uint64_t ni, const float4* __restrict__ inode, const float4* __restrict__ leaf0,
-    uint32_t* __restrict__ rest, uint32_t n_warps, uint32_t* __restrict__ n_rest,
-    unsigned long long* __restrict__ counts, uint32_t count_stride) {
+    uint32_t* __restrict__ rest, uint32_t n_warps, uint32_t* __restrict__ n_rest, uint8_t* __restrict__ done,
+    unsigned long long* __restrict__ tally, unsigned long long* __restrict__ counts, uint32_t count_stride) {
   __shared__ FastSmem smem[WARPS];
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
@@ -121,6 +125,20 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS_PER_SM / WARPS) k_wn_filter(
   const FastSignMesh M = meshes[mesh];
   const uint32_t i0 = act_base[mesh] + (span - span_base[mesh]) * span_size;
   const uint32_t nv = min(span_size, act_base[mesh + 1] - i0);
+  const uint32_t n_groups = (nv + 31) / 32;
+  // whether the filter has left too many of the mesh's groups to be worth its time
+  auto wasted = [&] {
+    const uint2 t = __ldcg(reinterpret_cast<const uint2*>(tally + mesh));  // groups tried, of them left
+    return __any_sync(FULLM, t.x >= TALLY_FROM && TALLY_SHARE * t.y > t.x && span % TALLY_SAMPLE != 0) != 0;
+  };
+  {
+    // Distances from any band voxel to any vertex or dipole centre of the mesh
+    // stay below R2_MAX, past which the bound does not hold, when the root's
+    // diameter and the band do.
+    const float r = (M.n_tri > 1 ? inode[5 * uint64_t(M.inode_base)] : leaf0[5 * uint64_t(M.tri_base)]).w;
+    const float reach = 2.0f * r + M.band;
+    if (!(reach * reach < R2_MAX) || wasted()) return;  // NaN too
+  }
   const float4* frec_i = frec0 + 4 * uint64_t(M.inode_base);
   const float4* frec_l = frec0 + 4 * (ni + M.tri_base);
   const float4* leaf = leaf0 + 5 * uint64_t(M.tri_base);
@@ -150,12 +168,6 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS_PER_SM / WARPS) k_wn_filter(
     brho = fmaxf(brho, dx * dx + dy * dy + dz * dz);
   }
   brho = sqrtf(__uint_as_float(__reduce_max_sync(FULLM, __float_as_uint(brho)))) * 1.00001f;
-  // Distances from any voxel to any vertex or dipole centre of the mesh stay
-  // below R2_MAX when the root's sphere and these voxels' do.
-  const float4 Proot = root >= 0 ? inode[5 * uint64_t(M.inode_base)] : leaf[0];
-  const float reach = Proot.w + (fabsf(Proot.x - bcx) + fabsf(Proot.y - bcy) + fabsf(Proot.z - bcz)) + brho;
-  const bool in_range = reach * reach < R2_MAX;  // false for NaN
-  const uint32_t n_groups = (nv + 31) / 32;
   // Work of the groups whose cut was walked to its end.  Every visit opens a
   // node, takes its far field or its solid angle, and opening gives two more:
   // (visits + 1) / 2 of a cut are not openings.
@@ -225,7 +237,9 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS_PER_SM / WARPS) k_wn_filter(
   // ---- groups: the traversal's 32 voxels ----
   float4* slot = sm.slot;
   const float thr4 = M.thresh * FOURPI;
-  for (uint32_t g = 0; g < n_groups; ++g) {
+  uint32_t g = 0;
+  for (; g < n_groups; ++g) {
+    if (g && wasted()) break;
     const bool ok = 32 * g + lane < nv;
     const uint32_t vox = act[i0 + (ok ? 32 * g + lane : nv - 1)];
     const int3 gr = grid(vox);
@@ -248,7 +262,7 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS_PER_SM / WARPS) k_wn_filter(
       taylor_clear(T);
       Lane s;
       s.w = s.mag = s.etri = 0.0f;
-      s.bad = !in_range;
+      s.bad = false;
       uint32_t n_add = 0, n_visit = 0, n_exact = 0;
       bool lost = false;  // no room for the cut
       int sp = 0, pos = 0;
@@ -401,11 +415,15 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS_PER_SM / WARPS) k_wn_filter(
       open_lanes = __ballot_sync(FULLM, mine && !settled);
       if (!open_lanes || lost) break;
     }
-    if (open_lanes && lane == 0)
-      rest[counted ? atomicAdd(n_rest, 1u) : n_warps - 1u - atomicAdd(n_rest + 1, 1u)] = i0 + 32 * g;
+    if (lane == 0) {
+      atomicAdd(tally + mesh, open_lanes ? (1ull << 32) + 1ull : 1ull);
+      if (open_lanes) rest[counted ? atomicAdd(n_rest, 1u) : n_warps - 1u - atomicAdd(n_rest + 1, 1u)] = i0 + 32 * g;
+    }
     __syncwarp();
   }
   if (lane == 0) {
+    done[span] = uint8_t(g);
+    atomicAdd(n_rest + 2, g);
     unsigned long long* c = counts + uint64_t(mesh) * count_stride;
     atomicAdd(c, (unsigned long long)c_visit);
     atomicAdd(c + 1, (unsigned long long)((c_visit + c_cuts) / 2 - c_exact));
@@ -438,12 +456,14 @@ uint32_t fast_sign_span(bs_ctx* ctx, uint64_t n_act) {
 void fast_sign(bs_ctx* ctx, const uint32_t* act, const uint32_t* d_act_base, const uint32_t* d_span_base,
                uint32_t span, uint32_t n_spans, int K, const FastSignMesh* d_meshes, const int4* origins, float* values,
                const float4* frec, uint64_t n_internal, const float4* inode, const float4* leaf, uint32_t* rest,
-               uint32_t n_warps, uint32_t* n_rest, unsigned long long* d_counts, uint32_t count_stride) {
+               uint32_t n_warps, uint32_t* n_rest, uint8_t* done, unsigned long long* d_tally,
+               unsigned long long* d_counts, uint32_t count_stride) {
   if (n_spans == 0) return;
 #define BS_WN_FILTER(W)                                                                                            \
   BS_KERNEL(ctx, "k_wn_sign", (k_wn_filter<W><<<(n_spans + W - 1) / W, 32 * W, 0, ctx->stream>>>(                                \
                                   act, d_act_base, d_span_base, span, K, d_meshes, origins, values, frec, n_internal,    \
-                                  inode, leaf, rest, n_warps, n_rest, d_counts, count_stride)))
+                                  inode, leaf, rest, n_warps, n_rest, done, d_tally, \
+                                  d_counts, count_stride)))
   if (ctx->tune_wn_warps == 2)
     BS_WN_FILTER(2);
   else if (ctx->tune_wn_warps == 8)

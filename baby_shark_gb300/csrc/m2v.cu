@@ -1557,8 +1557,14 @@ __global__ void __launch_bounds__(WN_THREADS) k_wn_sign_batch(const uint32_t* __
 
 // The warps that the filter (fast_sign.cu) did not settle, each by its first
 // index into act: n_rest[0] from rest[0] up, whose work is counted there, and
-// n_rest[1] from rest[n_warps - 1] down, counted here.
-__global__ void __launch_bounds__(WN_THREADS) k_wn_sign_rest(const uint32_t* __restrict__ act,
+// n_rest[1] from rest[n_warps - 1] down, counted here; then, unless it came to
+// all of them (n_rest[2] of n_warps), those from the done[s]-th of span s on.
+// These blocks take WN_WARPS neighbouring warps at a time, which share nodes in
+// L1 (n_rest[3]: how many were taken; warps by themselves, in strides of the
+// grid: 9.8 against 7.0 ms for a torus out of the filter's range).
+constexpr int REST_BLOCKS = 10;  // per SM
+
+__global__ void __launch_bounds__(WN_THREADS, REST_BLOCKS) k_wn_sign_rest(const uint32_t* __restrict__ act,
                                                              const uint32_t* __restrict__ act_base, int K,
                                                              const MeshInfo* __restrict__ mi,
                                                              const uint32_t* __restrict__ tri_base,
@@ -1568,18 +1574,38 @@ __global__ void __launch_bounds__(WN_THREADS) k_wn_sign_rest(const uint32_t* __r
                                                              const float4* __restrict__ inodes,
                                                              const float4* __restrict__ leaves, M2VStats* stats,
                                                              const uint32_t* __restrict__ rest, uint32_t n_warps,
-                                                             const uint32_t* __restrict__ n_rest) {
+                                                             uint32_t* n_rest,
+                                                             const uint8_t* __restrict__ done,
+                                                             const uint32_t* __restrict__ span_base, uint32_t span) {
   __shared__ int stk[WN_WARPS][WN_STACK];
+  __shared__ uint32_t taken;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const uint32_t n0 = n_rest[0], n = n0 + n_rest[1];
-  for (uint32_t r = blockIdx.x * WN_WARPS + w; r < n; r += gridDim.x * WN_WARPS) {
-    const uint64_t i0 = rest[r < n0 ? r : n_warps - 1 - (r - n0)], i = i0 + lane;
-    const int mesh = find_seg(act_base, K, i0);
-    const uint64_t a1 = act_base[mesh + 1];
+  auto walk = [&](int mesh, uint64_t i0, bool count) {
+    const uint64_t i = i0 + lane, a1 = act_base[mesh + 1];
     const MeshInfo M = mi[mesh];
     wn_warp<2>(act, i, i < a1, a1 - 1, origins, values, inodes + 5 * uint64_t(inode_base[mesh]),
                leaves + 5 * uint64_t(tri_base[mesh]), nullptr, nullptr, int(M.n_tri), M.h, M.beta, M.thresh,
-               stats + mesh, stk, r >= n0);
+               stats + mesh, stk, count);
+  };
+  const uint32_t n0 = n_rest[0], n = n0 + n_rest[1];
+  for (uint32_t r = blockIdx.x * WN_WARPS + w; r < n; r += gridDim.x * WN_WARPS) {
+    const uint32_t i0 = rest[r < n0 ? r : n_warps - 1 - (r - n0)];
+    walk(find_seg(act_base, K, i0), i0, r >= n0);
+  }
+  if (n_rest[2] == n_warps) return;
+  const uint32_t per = span / 32;  // warps of a span
+  const uint64_t n_all = uint64_t(span_base[K]) * per;
+  for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0) taken = atomicAdd(n_rest + 3, 1u);
+    __syncthreads();
+    const uint64_t it = uint64_t(taken) * WN_WARPS + w;
+    if (it - w >= n_all) break;
+    const uint32_t s = uint32_t(it / per), g = uint32_t(it % per);
+    if (it >= n_all || g < done[s]) continue;
+    const int mesh = find_seg(span_base, K, s);
+    const uint64_t i0 = act_base[mesh] + uint64_t(s - span_base[mesh]) * span + 32 * g;
+    if (i0 < act_base[mesh + 1]) walk(mesh, i0, true);
   }
 }
 
@@ -2180,7 +2206,8 @@ static std::vector<bs_volume*> batch_core(bs_ctx* ctx, const float* d_xyz, const
       if (!any3) {
         std::vector<FastSignMesh> fm(K);
         for (int m = 0; m < K; ++m)
-          fm[m] = FastSignMesh{inode_base[m], tri_base[m], mi[m].n_tri, mi[m].h, mi[m].beta, mi[m].thresh};
+          fm[m] = FastSignMesh{inode_base[m], tri_base[m], mi[m].n_tri, mi[m].h, mi[m].beta, mi[m].thresh,
+                               2.0f * float(mi[m].band + 4) * mi[m].h};
         d_fm = DBuf<FastSignMesh>(ctx, K);
         BS_CUDA(cudaMemcpyAsync(d_fm.p, fm.data(), K * sizeof(FastSignMesh), cudaMemcpyHostToDevice, ctx->stream));
         frec = DBuf<float4>(ctx, 4 * (2 * nt - uint64_t(K)));
@@ -2255,18 +2282,23 @@ static std::vector<bs_volume*> batch_core(bs_ctx* ctx, const float* d_xyz, const
                                   mi[0].h, mi[0].beta, mi[0].thresh, st.p)))
     const int ww = ctx->tune_wn_warps;
     if (!any3) {
-      DBuf<uint32_t> rest(ctx, n_warps + 2);  // listed warps, and their two numbers
-      BS_CUDA(cudaMemsetAsync(rest.p + n_warps, 0, 2 * sizeof(uint32_t), s));
+      DBuf<uint32_t> rest(ctx, n_warps + 4);  // listed warps, and the counts that k_wn_sign_rest reads
+      BS_CUDA(cudaMemsetAsync(rest.p + n_warps, 0, 4 * sizeof(uint32_t), s));
+      const uint64_t n_spans = span_base[K];  // a tally per mesh, then a byte per span
+      DBuf<unsigned long long> tally(ctx, K + (n_spans + 7) / 8);
+      uint8_t* done = reinterpret_cast<uint8_t*>(tally.p + K);
+      BS_CUDA(cudaMemsetAsync(tally.p, 0, K * sizeof(unsigned long long) + n_spans, s));
       static_assert(offsetof(M2VStats, wn_exact) == offsetof(M2VStats, wn_visits) + 16 && sizeof(M2VStats) % 8 == 0,
                     "the filter adds to three consecutive counters");
       fast_sign(ctx, act.p, act_base.p, d_wb.p + K + 1, span, span_base[K], K, d_fm.p, origins.p, values.p, frec.p,
-                nt - uint64_t(K), inode.p, leaf.p, rest.p, uint32_t(n_warps), rest.p + n_warps, &st.p->wn_visits,
-                uint32_t(sizeof(M2VStats) / 8));
+                nt - uint64_t(K), inode.p, leaf.p, rest.p, uint32_t(n_warps), rest.p + n_warps, done, tally.p,
+                &st.p->wn_visits, uint32_t(sizeof(M2VStats) / 8));
       int n_sm = 0;
       BS_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, ctx->device));
-      const unsigned grid = unsigned(std::min<uint64_t>(blocks(n_warps, WN_WARPS), uint64_t(n_sm) * 8));
+      const unsigned grid = unsigned(std::min<uint64_t>(blocks(n_warps, WN_WARPS), uint64_t(n_sm) * REST_BLOCKS));
       BS_KERNEL(ctx, "k_wn_sign_rest", (k_wn_sign_rest<<<grid, WN_THREADS, 0, s>>>(act.p, act_base.p, K, d_mi.p, d_tb.p, d_ib.p, origins.p,
-                                                                               values.p, inode.p, leaf.p, st.p, rest.p, uint32_t(n_warps), rest.p + n_warps)));
+                                                                               values.p, inode.p, leaf.p, st.p, rest.p, uint32_t(n_warps), rest.p + n_warps, done,
+                                                                               d_wb.p + K + 1, span)));
     } else if (K == 1) {
       if (ww == 2)
         BS_WN3(2);

@@ -41,8 +41,9 @@ def stages(run, names):
     return out, best
 
 
-@pytest.mark.parametrize("tree,name,most", [("reference", "out_of_range", HANDED_OVER), ("fast", "few_voxels", SETTLED),
-                                            ("fast", "edges", SETTLED)])
+@pytest.mark.parametrize("tree,name,most", [("reference", "out_of_range", HANDED_OVER),
+                                            ("fast", "out_of_range", HANDED_OVER),
+                                            ("fast", "few_voxels", SETTLED), ("fast", "edges", SETTLED)])
 def test_sign_pass_against_the_traversal(tree, name, most):
     v, f, h, band, beta = cases()[name]
 

@@ -3,7 +3,7 @@
 walks it: the certified filter, or the traversal where the filter has no room
 for the cut or is not used.  They equal the counters of WindingNumbers on the
 same tree at the same points (on the library's tree in the pass's order, 32
-points per cut)."""
+points per cut), and so do the signs."""
 import numpy as np
 import pytest
 
@@ -21,29 +21,33 @@ KEYS = {"fast": ("wn_warp_visits", "wn_far", "wn_exact"), "reference": ("wn_far"
 
 def cases():
     s = shapes()
-    out = {k: (*s[k], 2.0) for k in ("torus", "on_grid", "degenerate", "tiny", "out_of_range", "coarse", "few2")}
+    out = {k: (*s[k], 2.0, 0.2) for k in ("torus", "on_grid", "degenerate", "tiny", "out_of_range", "coarse", "few2")}
     # every node near: the pending nodes of 32 voxels outgrow the filter's stacks
-    out["all_near"] = (*synthetic.torus(1.0, 0.3, 400, 200, 0.02, seed=3), 0.2, 1, 500.0)
+    out["all_near"] = (*synthetic.torus(1.0, 0.3, 400, 200, 0.02, seed=3), 0.2, 1, 500.0, 0.2)
+    # a threshold at the outside's value: half of the groups cannot be settled,
+    # and after the first ones the filter gives the mesh up
+    out["outside_value"] = (*synthetic.torus(1.0, 0.3, 256, 128, 0.02, seed=3), 0.006, 3, 2.0, 0.0)
     return out
 
 
 @pytest.mark.parametrize("tree", ["reference", "fast"])
 @pytest.mark.parametrize("name", sorted(cases()))
 def test_counters_equal_the_traversal(name, tree):
-    v, f, h, band, beta = cases()[name]
-    vol = convert_fast([(v, f)], [(h, band)], beta, 0.2)[0] if tree == "fast" else \
-        convert_reference(v, f, h, band, beta, 0.2)
+    v, f, h, band, beta, thresh = cases()[name]
+    vol = convert_fast([(v, f)], [(h, band)], beta, thresh)[0] if tree == "fast" else \
+        convert_reference(v, f, h, band, beta, thresh)
     st = context().last_stats()
-    o, _, m = vol.export()
+    o, val, m = vol.export()
     li, k = np.nonzero(np.stack([unpack_mask(x) for x in m])[:, MORTON])
     vi = MORTON[k]
     pts = (o[li] + np.stack([vi >> 6, (vi >> 3) & 7, vi & 7], 1)).astype(np.float32) * np.float32(h)
     wn = bs.WindingNumbers.from_mesh((v, f), ctx=context(), tree=tree)
-    want = dict.fromkeys(KEYS[tree], 0)
+    want, w = dict.fromkeys(KEYS[tree], 0), []
     for i in range(0, len(pts), 1 << 19):  # larger sets are reordered
-        wn.approximate(pts[i:i + (1 << 19)], beta)
+        w.append(wn.approximate(pts[i:i + (1 << 19)], beta))
         got = context().last_stats()
         for key in want:
             want[key] += got[key]
     assert len(pts) > 0 and want["wn_far"] + want["wn_exact"] > 0
     assert {key: st[key] for key in want} == want
+    assert np.array_equal(np.signbit(val[li, vi]), ~(np.concatenate(w) < np.float32(thresh)))
