@@ -512,16 +512,22 @@ void ref_tree_sign(bs_ctx* ctx, const RefTrees& t, const uint32_t* act, const ui
   BS_KERNEL(ctx, "k_rt_sign", (k_rt_sign<W><<<unsigned(n_bricks), 32 * W, 0, s>>>(                                     \
                                   act, voff, d_leaf_base, K, d_meshes, origins, values, frec.p, int(t.nt), t.rad_i.p, \
                                   t.rad_l.p, t.tri.p, d_act_base, und.p, n_und.p, d_counters)))
-  if (ctx->tune_wn_warps == 2)
+  int n_sm = 0;
+  BS_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, ctx->device));
+  // A brick's warps take its groups in turn, so where the bricks are too few
+  // for the SMs' warps (24 each) they get more of them, up to one per group.
+  int warps_of = ctx->tune_wn_warps;
+  while (warps_of < 16 && n_bricks * 2 * warps_of <= uint64_t(n_sm) * 24) warps_of *= 2;
+  if (warps_of == 2)
     BS_RT_SIGN(2);
-  else if (ctx->tune_wn_warps == 8)
+  else if (warps_of == 8)
     BS_RT_SIGN(8);
+  else if (warps_of == 16)
+    BS_RT_SIGN(16);
   else
     BS_RT_SIGN(4);
 #undef BS_RT_SIGN
   const unsigned grid = ref_tree_sign_exact_grid(ctx, n_act);
-  int n_sm = 0;
-  BS_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, ctx->device));
   const uint32_t enough = std::min(grid * REF_SIGN_WARPS, unsigned(n_sm) * 32);
   BS_KERNEL(ctx, "k_undecided_warps",
             (k_undecided_warps<<<1, 32, 0, s>>>(n_und.p, 2 * K, enough, warps.p)));

@@ -62,3 +62,15 @@ def test_sign_pass_against_the_traversal(tree, name, most):
     _, theirs = stages(lambda: wn.approximate(pts, beta), ("k_rt_points", "k_wn_points"))
     print("%s %s: sign pass %.3f ms, traversal %.3f ms" % (tree, name, mine, theirs))
     assert 0 < mine <= most * theirs
+
+
+def test_few_bricks_get_more_warps():
+    """A hundred bricks, each with more groups of voxels than the context's four
+    warps: asking for eight warps a brick must not be what makes them fast."""
+    v, f = synthetic.torus(1.0, 0.3, 256, 128, 0.02, seed=3)
+    times = {}
+    for warps in (8, 4):  # four is a context's own
+        context().set_launch_shape(0, warps, 0)
+        _, times[warps] = stages(lambda: convert_reference(v, f, 0.05, 1, 4.0, 0.2), ("k_rt_sign",))
+    print("k_rt_sign %.3f ms with 4 warps, %.3f ms with 8" % (times[4], times[8]))
+    assert 0 < times[4] <= 1.2 * times[8]
