@@ -46,6 +46,7 @@ struct bs_ctx {
   int tune_dist_threads = 128;
   int tune_dist_batch = 32;  // sub-triangles per warp tile of the distance pass (8, 16, 32)
   int tune_wn_warps = 4;
+  bool dist_on_patches = false;  // the distance pass of the last mesh -> volume call
   // counters of the last mesh -> volume, offset or dual contouring call
   // (see bs_ctx_last_counters); [8] names the call that wrote them
   uint64_t last_stats[16] = {};

@@ -2082,6 +2082,7 @@ static std::vector<bs_volume*> batch_core(bs_ctx* ctx, const float* d_xyz, const
     uncullable += hst[m].n_uncullable;
   }
   const bool patches = area > 0.0 && est > PATCH_PAIRS * area && ns >= 2 * nt && PATCH_UNCULLABLE * uncullable <= ns;
+  ctx->dist_on_patches = patches;
   DBuf<Patch> pat;
   uint64_t n_list = ns;  // entries of the lists' kind: sub-triangles or patches
   if (patches) {
@@ -2606,7 +2607,10 @@ bs_status bs_winding_numbers_free(bs_wn_tree* t) {
 // and tiles of 8 / 16 / 32 sub-triangles per warp (8 shapes: 256 threads
 // take tiles of 8 or 16), the sign pass with 2 / 4 / 8 warps per block; two
 // rounds, best of each, and keeps the fastest of each pass for the context's
-// later calls.  h_choice: [threads per brick, warps per sign block, tile];
+// later calls.  The distance pass on patches has no tile: its three shapes are
+// timed, each time stands for all tiles, and the tile is left as it is (16 at
+// most with 256 threads).  Of the sign pass's a shape is taken for another only
+// when it is 2 % faster (with few bricks several are the same).  h_choice: [threads per brick, warps per sign block, tile];
 // h_ms (optional, 11 floats): the 8 distance shapes in the order (64, 8),
 // (64, 16), (64, 32), (128, 8), (128, 16), (128, 32), (256, 8), (256, 16),
 // then the sign pass with 2, 4, 8 warps.
@@ -2631,31 +2635,36 @@ bs_status bs_autotune_mesh_to_volume(bs_ctx* ctx, const float* d_xyz, uint64_t n
     for (double& b : best_d) b = 1e30;
     for (double& b : best_w) b = 1e30;
     bs::volume_release(bs::mesh_to_volume_impl(ctx, d_xyz, nv, d_tri, nt, *p));  // warm-up
+    const bool patches = ctx->dist_on_patches;
+    auto tile_of = [&](int c) { return !patches ? dist_cand[c][1] : dist_cand[c][0] == 256 ? std::min(db0, 16) : db0; };
     ctx->timing = true;
     for (int round = 0; round < 2; ++round) {
-      for (int c = 0; c < 8; ++c) {
+      for (int c = 0; c < 8; c += patches ? 3 : 1) {
+        const int w = patches ? c / 3 : c % 3;
         ctx->tune_dist_threads = dist_cand[c][0];
-        ctx->tune_dist_batch = dist_cand[c][1];
-        ctx->tune_wn_warps = wn_cand[c % 3];
+        ctx->tune_dist_batch = tile_of(c);
+        ctx->tune_wn_warps = wn_cand[w];
         ctx->stages.clear();
         bs::volume_release(bs::mesh_to_volume_impl(ctx, d_xyz, nv, d_tri, nt, *p));
         bs_ctx_resolve_stages(ctx);
         const auto d = ctx->stages.find("k_brick_distance");
-        auto w = ctx->stages.find("k_wn_sign");
-        if (w == ctx->stages.end()) w = ctx->stages.find("k_rt_sign");  // the reference's tree
-        if (d != ctx->stages.end()) best_d[c] = std::min(best_d[c], d->second.ms);
-        if (w != ctx->stages.end()) best_w[c % 3] = std::min(best_w[c % 3], w->second.ms);
+        auto sign = ctx->stages.find("k_wn_sign");
+        if (sign == ctx->stages.end()) sign = ctx->stages.find("k_rt_sign");  // the reference's tree
+        for (int k = c; d != ctx->stages.end() && k < (patches ? std::min(c + 3, 8) : c + 1); ++k)
+          best_d[k] = std::min(best_d[k], d->second.ms);
+        if (sign != ctx->stages.end()) best_w[w] = std::min(best_w[w], sign->second.ms);
       }
     }
-    int bd = 4, bw = 1;
+    int bd = 4, bw = ww0 == 2 ? 0 : ww0 == 8 ? 2 : 1;
     for (int c = 0; c < 8; ++c)
       if (best_d[c] < best_d[bd]) bd = c;
+    const double now_w = best_w[bw];
     for (int c = 0; c < 3; ++c)
-      if (best_w[c] < best_w[bw]) bw = c;
+      if (best_w[c] < best_w[bw] && best_w[c] < 0.98 * now_w) bw = c;
     ctx->stages = saved;
     ctx->timing = timing0;
     ctx->tune_dist_threads = dist_cand[bd][0];
-    ctx->tune_dist_batch = dist_cand[bd][1];
+    ctx->tune_dist_batch = tile_of(bd);
     ctx->tune_wn_warps = wn_cand[bw];
     h_choice[0] = ctx->tune_dist_threads;
     h_choice[1] = ctx->tune_wn_warps;

@@ -178,7 +178,10 @@ bs_status bs_mesh_to_volume_batch_device(bs_ctx* ctx, uint64_t n_meshes, const f
  * per brick and tiles of 8 / 16 / 32 sub-triangles per warp (256 threads take
  * tiles of 8 or 16), the sign pass with 2 / 4 / 8 warps per block, two rounds
  * — and keeps the fastest of each pass for the context's later conversions
- * (results do not depend on them).  h_choice[3]: the chosen threads per
+ * (results do not depend on them).  On a mesh whose distance pass works on
+ * patches of sub-triangles, which has no tile, the threads alone are timed, each
+ * time stands for all tiles, and the tile stays (16 at most with 256 threads);
+ * the sign warps change only for a gain of 2 %.  h_choice[3]: the chosen threads per
  * brick, warps per sign block and tile; h_ms (optional, 11 floats): the best
  * distance-pass times of the shapes (64, 8), (64, 16), (64, 32), (128, 8),
  * (128, 16), (128, 32), (256, 8), (256, 16), then the sign-pass times with
@@ -188,7 +191,8 @@ bs_status bs_autotune_mesh_to_volume(bs_ctx* ctx, const float* d_xyz, uint64_t n
                                      const bs_m2v_params* p, int32_t* h_choice, float* h_ms);
 /* Sets the launch shapes directly (0 keeps the current value; a context
  * starts at 128 threads per brick, tiles of 32 sub-triangles and 4 sign
- * warps, and a tile left at 0 with 256 threads becomes 16). */
+ * warps, and a tile left at 0 with 256 threads becomes 16; a mesh of a few
+ * hundred bricks takes up to 16 sign warps on the reference's tree). */
 bs_status bs_ctx_set_launch_shape(bs_ctx* ctx, int32_t dist_threads, int32_t wn_warps, int32_t dist_tile);
 /* ------------------------------------------------------------- volumes --- */
 /* Volume::with_voxel_size (volume/mod.rs:17-24): an empty volume (no leaves,

@@ -52,3 +52,20 @@ def test_slender_triangles_keep_the_pass_on_sub_triangles(aspect, patches):
     st = context().last_stats()
     assert (st["voxel_pairs_evaluated"] < st["voxel_pairs"]) == patches
     assert_same(vol, mesh, h, band)
+
+
+@pytest.mark.parametrize("tile", [8, 32])
+def test_autotune_keeps_the_tile_on_patches(tile):
+    """The pass on patches has no tile: what the context has must stay, and no
+    more than the three shapes be timed."""
+    ctx = bs.Context(0)
+    mesh = synthetic.torus(1.0, 0.3, 96, 48, 0.02, seed=5)
+    ctx.set_launch_shape(128, 4, tile)
+    assert convert(mesh, 0.02, 4, ctx)[1]
+    choice = ctx.autotune(mesh, 0.02, 4)
+    t = choice["distance_ms"]
+    assert choice["dist_tile"] == (min(tile, 16) if choice["dist_threads"] == 256 else tile)
+    assert t[64, 8] == t[64, 16] == t[64, 32] > 0 and t[128, 8] == t[128, 16] == t[128, 32] > 0
+    assert t[256, 8] == t[256, 16] > 0
+    assert t[choice["dist_threads"], 16] == min(t.values())
+    assert all(ms > 0 for ms in choice["sign_ms"].values())
