@@ -69,3 +69,18 @@ def test_autotune_keeps_the_tile_on_patches(tile):
     assert t[256, 8] == t[256, 16] > 0
     assert t[choice["dist_threads"], 16] == min(t.values())
     assert all(ms > 0 for ms in choice["sign_ms"].values())
+
+
+@pytest.mark.parametrize("band,patches", [(1, False), (4, True)])
+def test_every_launch_shape_of_both_passes_matches_oracle(band, patches):
+    ctx = bs.Context(0)
+    mesh, h = synthetic.torus(1.0, 0.3, 96, 48, 0.02, seed=5), 0.02
+    o, _, _ = ob.mesh_to_volume(*mesh, h, band)
+    o = o.export()
+    for threads, tile in ((64, 8), (64, 16), (64, 32), (128, 8), (128, 16), (128, 32), (256, 8), (256, 16)):
+        ctx.set_launch_shape(threads, 0, tile)
+        vol, took = convert(mesh, h, band, ctx)
+        assert took == patches
+        rep = compare_volumes(vol.export(), o, check_inactive=True)
+        assert rep["leaf_set_equal"] and rep["mask_mismatch_leaves"] == rep["value_mismatch"] == 0, rep
+        assert rep["sign_mismatch"] == rep["inactive_mismatch"] == 0 and rep["active"] > 0, rep
