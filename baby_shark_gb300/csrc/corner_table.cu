@@ -57,7 +57,8 @@ __device__ __forceinline__ uint32_t key_bits(float f) {
 // Every point finds or claims the slot of its coordinates in an open-addressing
 // table; a slot holds the smallest index of its points so far.  Which of the
 // equal points a comparison meets does not matter, so the outcome does not
-// depend on scheduling.  A NaN point equals nothing and takes no slot.
+// depend on scheduling.  A NaN point equals nothing and takes no slot.  The
+// hash mixes with the multipliers of MurmurHash3's 64-bit finaliser (Appleby).
 constexpr uint32_t NO_POINT = 0xffffffffu;
 
 __global__ void k_merge_insert(const float* __restrict__ p, uint64_t n, uint32_t* __restrict__ table, uint64_t mask,

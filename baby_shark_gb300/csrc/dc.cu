@@ -252,8 +252,6 @@ __global__ void __launch_bounds__(32 * DC_WARPS) k_dc_edge_points(DcVol V, uint6
 }
 
 // voxel/utils.rs:88-97 and dual_contouring.rs:410-423
-__constant__ int8_t c_cube[8][3] = {{0, 0, 0}, {1, 0, 0}, {1, 1, 0}, {0, 1, 0},
-                                    {0, 0, 1}, {1, 0, 1}, {1, 1, 1}, {0, 1, 1}};
 __constant__ int8_t c_edges[12][4] = {{0, 0, 0, 0}, {0, 0, 0, 1}, {0, 0, 0, 2}, {1, 0, 0, 1},
                                       {1, 0, 0, 2}, {0, 0, 1, 0}, {0, 0, 1, 1}, {0, 1, 0, 0},
                                       {0, 1, 0, 2}, {1, 0, 1, 1}, {0, 1, 1, 0}, {1, 1, 0, 2}};
@@ -562,8 +560,8 @@ __global__ void __launch_bounds__(32 * DC_WARPS) k_dc_quads(DcVol V, uint64_t n,
 // Launches shared with dc_noalloc.cu (tiles: the volume has active tiles).
 static inline unsigned dc_blocks(uint64_t n) { return unsigned((n + DC_WARPS - 1) / DC_WARPS); }
 
-void launch_dc_prepare(const DcVol& V, uint64_t n, int* nbr, uint32_t* sgn, cudaStream_t s) {
-  k_dc_neighbours<<<unsigned((27 * n + 255) / 256), 256, 0, s>>>(V.org, V.hash, n, nbr);
+void launch_dc_prepare(const DcVol& V, LeafHash hash, uint64_t n, int* nbr, uint32_t* sgn, cudaStream_t s) {
+  k_dc_neighbours<<<unsigned((27 * n + 255) / 256), 256, 0, s>>>(V.org, hash, n, nbr);
   k_dc_signs<<<dc_blocks(n), 32 * DC_WARPS, 0, s>>>(V.val, n, sgn);
 }
 void launch_dc_masks(bool tiles, const DcVol& V, uint64_t n, uint2* em, uint32_t* ccnt, uint2* cellm, uint32_t* cellc,
@@ -618,7 +616,7 @@ void dual_contour_impl(bs_ctx* ctx, bs_volume* v, float voxel_size, int mode) {
   hb.build(ctx, v->d_origins, n, n);
   DBuf<int> nbr(ctx, 27 * n);
   DBuf<uint32_t> sgn(ctx, 16 * n);
-  DcVol V{v->d_origins, v->d_values, v->d_masks, sgn.p, nbr.p, hb.h, TileLookup{}};
+  DcVol V{v->d_origins, v->d_values, v->d_masks, sgn.p, nbr.p, TileLookup{}};
   if (has_active_tiles(v)) {
     // The reference stops at active tiles (todo!(), dual_contouring.rs:139,
     // 186, 347).  Here the passes still visit the leaves only and read every
@@ -633,7 +631,7 @@ void dual_contour_impl(bs_ctx* ctx, bs_volume* v, float voxel_size, int mode) {
   DBuf<DcStats> st(ctx, 1);
   BS_CUDA(cudaMemsetAsync(st.p, 0, sizeof(DcStats), s));
   ctx->launches++;  // two kernels
-  BS_KERNEL(ctx, "k_dc_prepare", launch_dc_prepare(V, n, nbr.p, sgn.p, s));
+  BS_KERNEL(ctx, "k_dc_prepare", launch_dc_prepare(V, hb.h, n, nbr.p, sgn.p, s));
   // crossings and cells
   DBuf<uint2> em(ctx, n * 3 * 16), cellm(ctx, n * 16);
   DBuf<uint32_t> ccnt(ctx, n * 3 + 1), coff(ctx, n * 3 + 1), cellc(ctx, n + 1), celloff(ctx, n + 1);

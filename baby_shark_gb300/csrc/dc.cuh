@@ -13,7 +13,6 @@ struct DcVol {
   const uint32_t* msk;
   const uint32_t* sgn;  // [n][16] sign bits of the values
   const int* nbr;       // [n][27] neighbour leaves
-  LeafHash hash;
   TileLookup tiles;  // active tiles, read where a voxel lies outside every leaf (tiles.any == 0: none)
 };
 
@@ -23,7 +22,7 @@ struct DcStats {
 
 // The passes (tiles: the volume has active tiles, read through the tree's
 // `at`).  Masks come with ranks: (word, set bits in the words before it).
-void launch_dc_prepare(const DcVol& V, uint64_t n, int* nbr, uint32_t* sgn, cudaStream_t s);
+void launch_dc_prepare(const DcVol& V, LeafHash hash, uint64_t n, int* nbr, uint32_t* sgn, cudaStream_t s);
 void launch_dc_masks(bool tiles, const DcVol& V, uint64_t n, uint2* em, uint32_t* ccnt, uint2* cellm, uint32_t* cellc,
                      cudaStream_t s);
 void launch_dc_edge_points(bool tiles, const DcVol& V, uint64_t n, const uint2* em, const uint32_t* coff, float* pts,

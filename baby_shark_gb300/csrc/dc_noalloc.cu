@@ -255,8 +255,8 @@ extern "C" bs_status bs_dual_contour_noalloc(int device, void* stream, const int
     hash.mask = DCNA_HASH_CAP - 1;
     k_hash_insert<<<nblocks(n, 256), 256, 0, s>>>(hash, org, n, herr);
     BS_CUDA(cudaGetLastError());
-    DcVol V{org, d_values, d_masks, sgn, nbr, hash, tiles};
-    launch_dc_prepare(V, n, nbr, sgn, s);
+    DcVol V{org, d_values, d_masks, sgn, nbr, tiles};
+    launch_dc_prepare(V, hash, n, nbr, sgn, s);
     BS_CUDA(cudaGetLastError());
     launch_dc_masks(has_tiles, V, n, em, ccnt, cellm, cellc, s);
     BS_CUDA(cudaGetLastError());

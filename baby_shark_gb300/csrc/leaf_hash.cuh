@@ -16,6 +16,7 @@ __host__ __device__ __forceinline__ unsigned long long leaf_key(int x, int y, in
          static_cast<unsigned long long>(static_cast<uint32_t>((z >> 3) + (1 << 20)));
 }
 
+// MurmurHash3's 64-bit finaliser (Appleby).
 __device__ __forceinline__ uint32_t hash_slot(unsigned long long k, uint64_t mask) {
   k ^= k >> 33;
   k *= 0xff51afd7ed558ccdull;

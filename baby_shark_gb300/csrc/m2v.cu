@@ -1509,7 +1509,8 @@ __device__ __forceinline__ void wn_warp(const uint32_t* __restrict__ act, uint64
   }
 }
 
-template <int ORDER, int WARPS>
+// One mesh, order 3 (order 2 goes through the filter).
+template <int WARPS>
 __global__ void __launch_bounds__(32 * WARPS) k_wn_sign(const uint32_t* __restrict__ act, uint64_t na,
                                                         const int4* __restrict__ origins, float* __restrict__ values,
                                                         const float4* __restrict__ inode,
@@ -1521,7 +1522,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_wn_sign(const uint32_t* __restri
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const uint64_t i = (blockIdx.x * uint64_t(WARPS) + w) * 32 + lane;
   if ((blockIdx.x * uint64_t(WARPS) + w) * 32 >= na) return;  // whole warp out of range
-  wn_warp<ORDER>(act, i, i < na, na - 1, origins, values, inode, leaf, inode3, leaf3, n, h, beta, thresh, st, stk);
+  wn_warp<3>(act, i, i < na, na - 1, origins, values, inode, leaf, inode3, leaf3, n, h, beta, thresh, st, stk);
 }
 
 // Batches: warps are numbered per mesh (warp_base[m] .. warp_base[m+1]) so
@@ -2278,7 +2279,7 @@ static std::vector<bs_volume*> batch_core(bs_ctx* ctx, const float* d_xyz, const
   } else if (na > 0) {
     const uint64_t n_warps = warp_base[K];
 #define BS_WN3(WP)                                                                                              \
-  BS_KERNEL(ctx, "k_wn_sign", (k_wn_sign<3, WP><<<blocks(na, 32 * WP), 32 * WP, 0, s>>>(                      \
+  BS_KERNEL(ctx, "k_wn_sign", (k_wn_sign<WP><<<blocks(na, 32 * WP), 32 * WP, 0, s>>>(                      \
                                   act.p, na, origins.p, values.p, inode.p, leaf.p, inode3.p, leaf3.p, int(nt), \
                                   mi[0].h, mi[0].beta, mi[0].thresh, st.p)))
     const int ww = ctx->tune_wn_warps;

@@ -376,28 +376,26 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_patch_distance(
         bits &= ~((bd ? 2u : 1u) << (2 * (bi * cols + bj)));
       }
     }
+    // at most 8 per lane (a patch has nine sub-triangles, the nearest is taken),
+    // which PATCH_QUEUE has room for beside fewer than 32 left over
     const int n = __popc(bits);
     if (__any_sync(0xffffffffu, n)) {
-      // at most 17 per lane: room is made below 32 before each block of 8
-      while (__any_sync(0xffffffffu, bits)) {
-        const int take = min(__popc(bits), 8);
-        int pos = take;
+      int pos = n;
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-          const int v = __shfl_up_sync(0xffffffffu, pos, d);
-          if (lane >= d) pos += v;
-        }
-        const int added = __shfl_sync(0xffffffffu, pos, 31);
-        pos += qn2 - take;
-        for (int k = 0; k < take; ++k) {
-          const int c = __ffs(bits) - 1;
-          bits &= bits - 1u;
-          const int cell = c >> 1, i = cell / cols, j = cell - i * cols;
-          Q2[pos++] = make_uint2(off + sub_index(r0 + i, k0 + j, c & 1), uint32_t(o) | (outer ? 512u : 0u));
-        }
-        qn2 += added;
-        while (qn2 >= 32) drain2(32);
+      for (int d = 1; d < 32; d <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, pos, d);
+        if (lane >= d) pos += v;
       }
+      const int added = __shfl_sync(0xffffffffu, pos, 31);
+      pos += qn2 - n;
+      while (bits) {
+        const int c = __ffs(bits) - 1;
+        bits &= bits - 1u;
+        const int cell = c >> 1, i = cell / cols, j = cell - i * cols;
+        Q2[pos++] = make_uint2(off + sub_index(r0 + i, k0 + j, c & 1), uint32_t(o) | (outer ? 512u : 0u));
+      }
+      qn2 += added;
+      while (qn2 >= 32) drain2(32);
     }
   };
 

@@ -19,7 +19,7 @@ struct Level {
   float* d_tile = nullptr;        // [n][slots]
   uint8_t* d_first_neg = nullptr; // [n] first_value_sign() == Negative (after a flood fill)
   uint8_t* d_last_neg = nullptr;  // [n] last_value_sign() == Negative
-  std::vector<int4> h_key;        // host copy of d_key
+  std::vector<int4> h_key;        // host copy of d_key (L2 alone: the root level is decided on the host)
   Level() {}
   Level(int l, int cs) : log2(l), child_shift(cs), slots(1 << (3 * l)) {}
   void alloc(bs_ctx* ctx, uint64_t count);
