@@ -460,7 +460,7 @@ void fast_sign(bs_ctx* ctx, const uint32_t* act, const uint32_t* d_act_base, con
                unsigned long long* d_counts, uint32_t count_stride) {
   if (n_spans == 0) return;
 #define BS_WN_FILTER(W)                                                                                            \
-  BS_KERNEL(ctx, "k_wn_sign", (k_wn_filter<W><<<(n_spans + W - 1) / W, 32 * W, 0, ctx->stream>>>(                                \
+  BS_KERNEL(ctx, "k_wn_filter", (k_wn_filter<W><<<(n_spans + W - 1) / W, 32 * W, 0, ctx->stream>>>(                                \
                                   act, d_act_base, d_span_base, span, K, d_meshes, origins, values, frec, n_internal,    \
                                   inode, leaf, rest, n_warps, n_rest, done, d_tally, \
                                   d_counts, count_stride)))

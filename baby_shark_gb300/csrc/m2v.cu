@@ -2104,7 +2104,7 @@ static std::vector<bs_volume*> batch_core(bs_ctx* ctx, const float* d_xyz, const
   DBuf<uint32_t> cnt(ctx, DC + 1), pair_off(ctx, DC + 1), flag(ctx, D + 1), bidx(ctx, D + 1);
   BS_CUDA(cudaMemsetAsync(cnt.p, 0, (DC + 1) * sizeof(uint32_t), s));
   if (patches)
-    BS_KERNEL(ctx, "k_count_pairs", (k_count_patches<<<blocks(n_list, 256), 256, 0, s>>>(pat.p, n_list, S.p, d_dirs.p, d_db.p, cnt.p, st.p)));
+    BS_KERNEL(ctx, "k_count_patches", (k_count_patches<<<blocks(n_list, 256), 256, 0, s>>>(pat.p, n_list, S.p, d_dirs.p, d_db.p, cnt.p, st.p)));
   else
     BS_KERNEL(ctx, "k_count_pairs", (k_count_pairs<<<blocks(ns, 256), 256, 0, s>>>(S.p, ns, d_dirs.p, d_db.p, cnt.p, st.p)));
   exclusive_scan(ctx, cnt.p, pair_off.p, DC + 1);
@@ -2143,7 +2143,7 @@ static std::vector<bs_volume*> batch_core(bs_ctx* ctx, const float* d_xyz, const
     pair_off.reset();
     bidx.reset();
     if (patches)
-      BS_KERNEL(ctx, "k_fill_pairs", (k_fill_patches<<<blocks(n_list, 256), 256, 0, s>>>(pat.p, n_list, S.p, d_dirs.p, d_db.p, cnt.p, list.p)));
+      BS_KERNEL(ctx, "k_fill_patches", (k_fill_patches<<<blocks(n_list, 256), 256, 0, s>>>(pat.p, n_list, S.p, d_dirs.p, d_db.p, cnt.p, list.p)));
     else
       BS_KERNEL(ctx, "k_fill_pairs", (k_fill_pairs<<<blocks(ns, 256), 256, 0, s>>>(S.p, ns, d_dirs.p, d_db.p, cnt.p, list.p)));
     cnt.reset();
@@ -2154,7 +2154,7 @@ static std::vector<bs_volume*> batch_core(bs_ctx* ctx, const float* d_xyz, const
                                                                                             leaf_base.p, K, values.p, \
                                                                                             masks.p, st.p)))
 #define BS_PATCH(TH)                                                                                                 \
-  BS_KERNEL(ctx, "k_brick_distance", (k_patch_distance<TH><<<unsigned(nb), TH, 0, s>>>(origins.p, list_off.p,      \
+  BS_KERNEL(ctx, "k_patch_distance", (k_patch_distance<TH><<<unsigned(nb), TH, 0, s>>>(origins.p, list_off.p,      \
                                                                                         list.p, pat.p, S.p, d_mi.p,  \
                                                                                         leaf_base.p, K, values.p,    \
                                                                                         masks.p, st.p)))
@@ -2309,7 +2309,7 @@ static std::vector<bs_volume*> batch_core(bs_ctx* ctx, const float* d_xyz, const
       else
         BS_WN3(4);
     } else {
-      BS_KERNEL(ctx, "k_wn_sign", (k_wn_sign_batch<<<blocks(n_warps, WN_WARPS), WN_THREADS, 0, s>>>(act.p, act_base.p, d_wb.p, K, d_mi.p, d_tb.p,
+      BS_KERNEL(ctx, "k_wn_sign_batch", (k_wn_sign_batch<<<blocks(n_warps, WN_WARPS), WN_THREADS, 0, s>>>(act.p, act_base.p, d_wb.p, K, d_mi.p, d_tb.p,
                                                                                        d_ib.p, origins.p, values.p, inode.p, leaf.p,
                                                                                        inode3.p, leaf3.p, st.p)));
     }
@@ -2648,9 +2648,10 @@ bs_status bs_autotune_mesh_to_volume(bs_ctx* ctx, const float* d_xyz, uint64_t n
         ctx->stages.clear();
         bs::volume_release(bs::mesh_to_volume_impl(ctx, d_xyz, nv, d_tri, nt, *p));
         bs_ctx_resolve_stages(ctx);
-        const auto d = ctx->stages.find("k_brick_distance");
-        auto sign = ctx->stages.find("k_wn_sign");
-        if (sign == ctx->stages.end()) sign = ctx->stages.find("k_rt_sign");  // the reference's tree
+        const auto d = ctx->stages.find(patches ? "k_patch_distance" : "k_brick_distance");
+        auto sign = ctx->stages.find("k_rt_sign");  // the reference's tree
+        for (const char* fast : {"k_wn_filter", "k_wn_sign"})
+          if (sign == ctx->stages.end()) sign = ctx->stages.find(fast);
         for (int k = c; d != ctx->stages.end() && k < (patches ? std::min(c + 3, 8) : c + 1); ++k)
           best_d[k] = std::min(best_d[k], d->second.ms);
         if (sign != ctx->stages.end()) best_w[w] = std::min(best_w[w], sign->second.ms);

@@ -68,9 +68,8 @@ WN_EXACT_PER_VOXEL = 14.96  # (1,048,576 triangles) from the 4.5 M band voxels o
 WN_FLOP_PER_VOXEL = int(round(WN_FAR_PER_VOXEL * WN_FLOP_FAR + WN_EXACT_PER_VOXEL * WN_FLOP_EXACT))
 # dram__bytes_read.sum + dram__bytes_write.sum per launch from one ncu capture of
 # one full torus (35,589,878 band voxels: k_rt_sign 526 + 167 MB, the distance
-# pass on patches 1,168 + 266 MB) and of a scan with holes (14,745,700 band
-# voxels: the fast tree's pass 399 + 70 MB, scaled by the voxels)
-TRAFFIC_PER_LAUNCH = {"k_wn_sign": 1134e6, "k_brick_distance": 1433e6, "k_rt_sign": 693e6}
+# pass on patches 1,168 + 266 MB)
+TRAFFIC_PER_LAUNCH = {"k_patch_distance": 1433e6, "k_rt_sign": 693e6}
 # smsp__inst_executed.sum per launch of the same capture of k_rt_sign: warp
 # instructions, the kernel's real bound (it issues on 70 % of the cycles);
 # scaled by the voxels of a launch
@@ -396,7 +395,7 @@ def run_ours(args):
     per_launch_s = tot_ms / nl / 1000.0
     # stats are of the last conversion (torus B); both tori are the same size class
     extra = {}
-    if name == "k_brick_distance":
+    if name in ("k_brick_distance", "k_patch_distance"):
         ev = stats["voxel_pairs_evaluated"]
         # the culls are per patch and sub-triangle where patches are used: not counted
         flops = FLOP_PER_PAIR * ev
@@ -423,7 +422,7 @@ def run_ours(args):
                 "peak_per_s": issue_peak, "frac": inst / per_launch_s / issue_peak,
                 "source": "smsp__inst_executed.sum of one ncu capture (profiles/k_rt_sign_one_torus.md), per band "
                           "voxel; peak = 152 SMs x 4 schedulers x the sampled SM clock"}
-    elif name == "k_wn_sign":
+    elif name in ("k_wn_filter", "k_wn_sign"):
         flops = WN_FLOP_PER_VOXEL * stats["active_voxels"]
         algo = ("%d FLOP per band voxel (the reference's own traversal: %.0f far-field nodes x %d FLOP + "
                 "%.0f exact triangles x %d FLOP, counted by the oracle) x %d voxels per launch"

@@ -1,6 +1,6 @@
 """Which distance pass a conversion takes (csrc/m2v.cu: on patches of
 sub-triangles where a band voxel meets many of their boxes and they can be
-culled, else on sub-triangles; the stage k_patches runs for the first alone)."""
+culled, else on sub-triangles; the timed stages carry the kernels' names)."""
 import numpy as np
 import pytest
 
@@ -31,7 +31,12 @@ def convert(mesh, h, band, ctx=None):
     try:
         ctx.stage_times(reset=True)
         vol = bs.MeshToVolume(ctx).with_voxel_size(h).with_narrow_band_width(band).convert(mesh)
-        return vol, "k_patches" in ctx.stage_times(reset=True)
+        st = ctx.stage_times(reset=True)
+        took = "k_patches" in st
+        for sub, patch in (("k_brick_distance", "k_patch_distance"), ("k_count_pairs", "k_count_patches"),
+                           ("k_fill_pairs", "k_fill_patches")):
+            assert (patch in st) == took and (sub in st) != took
+        return vol, took
     finally:
         ctx.set_stage_timing(False)
 

@@ -52,7 +52,8 @@ def test_sign_pass_against_the_traversal(tree, name, most):
             return convert_fast([(v, f)], [(h, band)], beta, 0.2)[0]
         return convert_reference(v, f, h, band, beta, 0.2)
 
-    vol, mine = stages(convert, ("k_rt_sign", "k_undecided_warps", "k_rt_sign_exact", "k_wn_sign", "k_wn_sign_rest"))
+    vol, mine = stages(convert, ("k_rt_sign", "k_undecided_warps", "k_rt_sign_exact", "k_wn_sign", "k_wn_filter",
+                                   "k_wn_sign_rest"))
     o, _, m = vol.export()
     li, k = np.nonzero(np.stack([unpack_mask(x) for x in m])[:, MORTON])
     vi = MORTON[k]
