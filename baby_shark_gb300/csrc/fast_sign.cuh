@@ -17,8 +17,8 @@ void fast_filter_records(bs_ctx* ctx, const float4* inode, uint64_t n_internal, 
                          const float4* leaf, uint64_t nt, const uint32_t* d_tri_base, int K,
                          const FastSignMesh* d_meshes, float4* frec);
 
-// Squared distance of the traversal's far test, the same float32 operations
-// wherever a cut is taken.
+// Squared distance of the far test of the order-2 traversal, the same float32
+// operations wherever its cut is taken (the order-3 traversal has no filter).
 __device__ __forceinline__ float cut_dist2(float rx, float ry, float rz) {
   return __fmaf_rn(rz, rz, __fmaf_rn(rx, rx, __fmul_rn(ry, ry)));
 }

@@ -1409,7 +1409,7 @@ __device__ __forceinline__ float wn_traverse(F3 q, const float4* __restrict__ in
     if (node >= 0) {
       const float4 P = inode[5 * node];
       const float rx = P.x - q.x, ry = P.y - q.y, rz = P.z - q.z;
-      const float r2 = cut_dist2(rx, ry, rz);
+      const float r2 = ORDER >= 3 ? rx * rx + ry * ry + rz * rz : cut_dist2(rx, ry, rz);
       if (!__all_sync(0xffffffffu, r2 > P.w * P.w * beta2)) return true;
       const float4 A = inode[5 * node + 1], B0 = inode[5 * node + 2], B1 = inode[5 * node + 3],
                    B2 = inode[5 * node + 4];
@@ -1430,7 +1430,7 @@ __device__ __forceinline__ float wn_traverse(F3 q, const float4* __restrict__ in
     const int li = ~node;
     const float4 P = leaf[5 * li];
     const float rx = P.x - q.x, ry = P.y - q.y, rz = P.z - q.z;
-    const float r2 = cut_dist2(rx, ry, rz);
+    const float r2 = ORDER >= 3 ? rx * rx + ry * ry + rz * rz : cut_dist2(rx, ry, rz);
     float wv;
     if (__all_sync(0xffffffffu, r2 > P.w * P.w * beta2)) {
       const float4 A = leaf[5 * li + 1];

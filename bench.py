@@ -618,7 +618,7 @@ def variant_secondary(ctx, params, dev, L, N, bs, C, args, tree=1, order=2, beta
         diff += int(np.sum(np.signbit(va[act]) != np.signbit(vb[act])))
     return {"value": band / (min(ms) / 1000.0), "unit": UNIT, "ms_per_step": min(ms),
             "sign_differences_vs_headline": diff, "band_voxels": int(band),
-            "tree": "PLOC (warp-coherent traversal)" if tree == 1 else "reference SAH", "order": order, "beta": beta}
+            "tree": "PLOC" if tree == 1 else "reference SAH", "order": order, "beta": beta}
 
 
 def learned_secondary(ctx, v, f, n_q, steps=2, warmup=1, validation=200000, seed=12345):
