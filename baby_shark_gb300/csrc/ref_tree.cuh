@@ -68,14 +68,15 @@ void ref_tree_sign(bs_ctx* ctx, const RefTrees& t, const uint32_t* act, const ui
 // voxels from list[d_act_base[m] + 32 d_leaf_base[m]] up, whose work the
 // counters have, and d_count[2 m + 1] that end before the next mesh's, whose
 // work is added (NO_VOXEL entries are passed over); list l in warps d_warps[l]
-// .. d_warps[l + 1] of d_warps[2 K + 1] voxels each (device arrays).  grid:
+// .. d_warps[l + 1] of d_warps[2 K + 1] voxels each, d_warps[2 K + 2] zero
+// (device arrays).  grid:
 // blocks of REF_SIGN_WARPS warps for at most max_list voxels.
 constexpr int REF_SIGN_WARPS = 4;
 constexpr uint32_t NO_VOXEL = 0xffffffffu;  // bricks are fewer than 2^23
 unsigned ref_tree_sign_exact_grid(bs_ctx* ctx, uint64_t max_list);
 void ref_tree_sign_exact(bs_ctx* ctx, const RefTrees& t, unsigned grid, const uint32_t* list,
                          const uint32_t* d_act_base, const uint32_t* d_leaf_base, const uint32_t* d_count,
-                         const uint32_t* d_warps, int K, const RefSignMesh* d_meshes, const int4* origins, float* values,
+                         uint32_t* d_warps, int K, const RefSignMesh* d_meshes, const int4* origins, float* values,
                          unsigned long long* d_counters);
 
 // WindingNumbers::approximate (aabb_tree.rs:654-660) at np device points of

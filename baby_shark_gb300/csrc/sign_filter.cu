@@ -467,10 +467,11 @@ __global__ void __launch_bounds__(32 * WARPS) k_rt_sign(
 }
 
 // Work split of the exact pass over n lists: base[l] = first warp of list l,
-// base[n + 1] = voxels per warp.  A warp walks the union of its voxels' cuts,
-// and the few undecided voxels are scattered over the mesh, so as long as warps
-// are free a warp takes fewer voxels (one, when n_warps suffice for all).  A
-// power of two, which keeps 32 voxels that were listed together together.
+// base[n + 1] = voxels per warp, base[n + 2] = 0.  A warp walks the union of its
+// voxels' cuts, and the few undecided voxels are scattered over the mesh, so as
+// long as warps are free a warp takes fewer voxels (one, when n_warps suffice
+// for all).  A power of two, which keeps 32 voxels that were listed together
+// together.
 __global__ void k_undecided_warps(const uint32_t* __restrict__ n_undecided, int n, uint32_t n_warps,
                                   uint32_t* __restrict__ base) {
   const int lane = threadIdx.x;
@@ -493,6 +494,7 @@ __global__ void k_undecided_warps(const uint32_t* __restrict__ n_undecided, int 
   if (lane == 0) {
     base[n] = at;
     base[n + 1] = per;
+    base[n + 2] = 0;
   }
 }
 
@@ -503,7 +505,7 @@ void ref_tree_sign(bs_ctx* ctx, const RefTrees& t, const uint32_t* act, const ui
                    const RefSignMesh* d_meshes, const int4* origins, float* values, unsigned long long* d_counters) {
   if (n_act == 0) return;
   cudaStream_t s = ctx->stream;
-  DBuf<uint32_t> und(ctx, n_act + 32 * n_bricks), n_und(ctx, 2 * K), warps(ctx, 2 * K + 2);
+  DBuf<uint32_t> und(ctx, n_act + 32 * n_bricks), n_und(ctx, 2 * K), warps(ctx, 2 * K + 3);
   DBuf<float4> frec(ctx, 8 * t.nt);
   BS_CUDA(cudaMemsetAsync(n_und.p, 0, 2 * K * sizeof(uint32_t), s));
   BS_KERNEL(ctx, "k_rt_filter_records", (k_rt_filter_records<<<unsigned((t.nt + 255) / 256), 256, 0, s>>>(
