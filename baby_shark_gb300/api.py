@@ -339,7 +339,7 @@ class MeshToVolume:
     def with_sign_tree(self, tree):
         """Tree of the sign pass: "reference" (default; the reference's SAH
         tree and summation order, bit-exact signs) or "fast" (the library's
-        PLOC tree with a warp-coherent traversal)."""
+        PLOC tree, one cut of it for 32 voxels)."""
         if tree not in ("reference", "fast"):
             raise ValueError("tree must be 'reference' or 'fast'")
         self.params.wn_tree = 0 if tree == "reference" else 1

@@ -28,9 +28,11 @@ using namespace sign_filter;
 constexpr int FRONT = 448;   // nodes a warp's first phase leaves to its groups
 constexpr int STACK = 256;   // pending nodes
 constexpr float E_GROUP = 0.02f;  // truncation error of one expanded node in a group's first attempt
-// A mesh of whose groups the filter has left more than one in TALLY_SHARE (it
-// takes about 0.4 of the traversal's time, twice that with the second attempt)
-// goes to the traversal from there on, but for one span in TALLY_SAMPLE.
+// A mesh of whose groups the filter has left more than one in TALLY_SHARE goes
+// to the traversal from there on, but for one span in TALLY_SAMPLE.  The filter
+// takes about 0.4 of the traversal's time, twice that with the second attempt,
+// so it pays below a third: with 40 % left (a torus, threshold 0) 11.5 ms with it
+// and 8.8 given up; below the line (20 k needles) 53.9 with it, 73.2 without.
 constexpr uint32_t TALLY_FROM = 64, TALLY_SHARE = 3, TALLY_SAMPLE = 32;
 constexpr int SLOT = 5;      // float4 per lane's broadcast slot: 4 and one that keeps the banks apart
 // the float32 squared distances are within 4 u: outside of this the traversal's test is certain
@@ -96,12 +98,13 @@ struct FastSmem {  // of a warp
   float taylor[11];  // the span's polynomial
 };
 
-// Every warp takes a span of voxels by itself.  Issue-bound: about 16 k
-// instructions per 32 voxels, of which the far fields per voxel (125 nodes)
-// take a quarter and the tests, the polynomials and the triangles (17) a fifth
-// each.  On a scan of 1.2 M triangles with holes and 14.7 M band voxels: 13.8
-// ms with the traversal of every warp, 8.1 ms here, 0.37 ms of it the
-// traversal of the warps left over.  Blocks that share one first phase behind
+// Every warp takes a span of voxels by itself.  Issue-bound: about 12 k
+// instructions per 32 voxels on a torus of 1 M triangles (35.7 M band voxels,
+// 15.0 ms), of which the far fields per voxel take a quarter and the tests, the
+// polynomials and the triangles (27) a fifth each.  On a scan of 1.2 M triangles
+// with holes and 14.7 M band voxels: 13.8 ms with the traversal of every warp,
+// 8.1 ms here, 0.37 ms of it the traversal of the warps left over.  80 registers
+// without a spill: 36 spilled bytes took 10 % longer.  Blocks that share one first phase behind
 // a barrier: 9.1 ms; spans of 64, 128, 512 voxels: +0.6, +0.1, +0.2 ms; 28 or
 // 32 warps per SM with spills: +0.1, +0.2 ms; testing a node with a vote of
 // all voxels instead of in a loop over them on its lane: +0.6 ms; E_GROUP
@@ -444,7 +447,8 @@ void fast_filter_records(bs_ctx* ctx, const float4* inode, uint64_t n_internal, 
 // Consecutive active voxels of a mesh that one warp takes, for n_act of them in
 // all: 32, 64, 128 or 256.  The longer a span, the more its groups share; but
 // a warp takes its groups one after another, so the spans must fill the SMs
-// several times over.
+// several times over (1, 2, 4, 8 times: 1.34, 1.21, 1.19, 1.23 ms for 1 M voxels;
+// 1,944 voxels of an icosphere: 0.51 ms in spans of 256, 0.12 of 32).
 uint32_t fast_sign_span(bs_ctx* ctx, uint64_t n_act) {
   int n_sm = 0;
   BS_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, ctx->device));

@@ -237,10 +237,10 @@ __global__ void k_fill_patches(const Patch* __restrict__ P, uint64_t np, const S
 // nearer; these are evaluated 32 at a time too.  A sub-triangle counts only
 // where its own widened box holds the voxel.
 //
-// Issue-bound (78 % of cycles issue): 10.9 G warp instructions and 12.2 ms on a
-// torus of 1 M triangles, 10.7 M sub-triangles and 35.6 M band voxels, where
-// the pass over sub-triangles takes 16.8 G and 15.6 ms; it evaluates 12 exact
-// distances per voxel instead of 28.  (Work units of 64 voxels with their own
+// Issue-bound (83 % of cycles issue): 10.9 G warp instructions and 12.0 ms
+// beside the tree build (10.5 alone) on a torus of 1 M triangles, 10.7 M
+// sub-triangles and 35.7 M band voxels, where the pass over sub-triangles takes
+// 16.8 G and 15.6 ms; it evaluates 12 exact distances per voxel instead of 28.  (Work units of 64 voxels with their own
 // nearest-first order: no fewer evaluations, 15.5 G instructions, 19.0 ms.)
 //
 // Threads per brick: 64, 128 or 256 (bs_autotune_mesh_to_volume); a warp

@@ -118,12 +118,13 @@ __device__ __noinline__ void hand_over(const uint32_t* __restrict__ act, uint32_
 
 // One CTA per brick: its first warp runs the brick's phase, then every warp
 // takes the next 32 voxels.  Issue-bound (like the exact traversal): 62.6 ms
-// with the exact traversal of every voxel, 15.1 ms here, on a torus of 1 M
+// with the exact traversal of every voxel, 15.2 ms here, on a torus of 1 M
 // triangles and 35.6 M band voxels; 38.2 and 10.4 ms on a scan of 1.2 M
 // triangles with holes and 19.2 M band voxels, 0.25 ms of it the exact pass
 // over 0.02 % of the voxels (0.3 % and 2.8 ms without the second attempt).
 // E_MAX between 0.03 and 0.06 changes it by 1 %; 0.1 spends the second
-// attempt on 3 to 16 % of the voxels.
+// attempt on 3 to 16 % of the voxels.  80 registers and a few spilled bytes, as
+// the compiler chooses; held to other numbers it took 1 to 7 % longer.
 template <int WARPS>
 __global__ void __launch_bounds__(32 * WARPS) k_rt_sign(
     const uint32_t* __restrict__ act, const uint32_t* __restrict__ voff, const uint32_t* __restrict__ leaf_base, int K,
@@ -517,7 +518,9 @@ void ref_tree_sign(bs_ctx* ctx, const RefTrees& t, const uint32_t* act, const ui
   int n_sm = 0;
   BS_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, ctx->device));
   // A brick's warps take its groups in turn, so where the bricks are too few
-  // for the SMs' warps (24 each) they get more of them, up to one per group.
+  // for the SMs' warps (24 each) they get more of them, up to one per group: 124
+  // bricks with 4, 8, 16 warps 8.7, 5.0, 3.5 ms (accuracy scale 8); 947 bricks
+  // with 4, 8 warps 0.70, 0.73 ms.
   int warps_of = ctx->tune_wn_warps;
   while (warps_of < 16 && n_bricks * 2 * warps_of <= uint64_t(n_sm) * 24) warps_of *= 2;
   if (warps_of == 2)

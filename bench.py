@@ -67,13 +67,13 @@ WN_EXACT_PER_VOXEL = 14.96  # (1,048,576 triangles) from the 4.5 M band voxels o
 #                             counts per band voxel (oracle/traversal_counts.py)
 WN_FLOP_PER_VOXEL = int(round(WN_FAR_PER_VOXEL * WN_FLOP_FAR + WN_EXACT_PER_VOXEL * WN_FLOP_EXACT))
 # dram__bytes_read.sum + dram__bytes_write.sum per launch from one ncu capture of
-# one full torus (35,589,878 band voxels: k_rt_sign 526 + 167 MB, the distance
-# pass on patches 1,168 + 266 MB)
-TRAFFIC_PER_LAUNCH = {"k_patch_distance": 1433e6, "k_rt_sign": 693e6}
+# one full torus (35,719,037 band voxels: k_rt_sign 527 + 168 MB, the distance
+# pass on patches 1,168 + 266 MB, the fast tree's filter 581 + 170 MB)
+TRAFFIC_PER_LAUNCH = {"k_patch_distance": 1433e6, "k_rt_sign": 695e6, "k_wn_filter": 750e6}
 # smsp__inst_executed.sum per launch of the same capture of k_rt_sign: warp
 # instructions, the kernel's real bound (it issues on 70 % of the cycles);
 # scaled by the voxels of a launch
-RT_SIGN_WARP_INST_PER_VOXEL = 13.23e9 / 35589878
+RT_SIGN_WARP_INST_PER_VOXEL = 13.36e9 / 35719037
 SM_COUNT_GB300 = 152
 SCHEDULERS_PER_SM = 4
 METRIC = "band voxels/s mesh→SDF+sign: learned/batched vs plain GPU, 0 sign flips"
@@ -580,7 +580,7 @@ def variant_secondary(ctx, params, dev, L, N, bs, C, args, tree=1, order=2, beta
     """The same conversion with another sign tree / far-field order /
     accuracy scale: band voxels/s, and how many band voxel signs differ from
     the headline (the reference's tree, order 2, scale 2).  tree 1 is the
-    library's PLOC tree with its warp-coherent traversal."""
+    library's PLOC tree."""
     import copy
 
     import torch

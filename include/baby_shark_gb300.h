@@ -90,7 +90,8 @@ bs_status bs_ctx_last_stats(const bs_ctx* ctx, uint64_t* out8);
  * mesh -> volume call evaluated after culling (the rest provably could not
  * lower their voxel's minimum), [10] far-field evaluations and [11] exact
  * solid angles of the winding-number pass in 64 bits (per voxel or point on
- * the reference's tree, per warp on the library's PLOC tree), [12] which tree
+ * the reference's tree, per warp on the library's PLOC tree; every cut once,
+ * whichever kernel walks it), [12] which tree
  * (0 the reference's, 1 PLOC), [13] and [14] on the reference's tree the
  * far-field evaluations and solid angles as the pass runs them (once for a
  * whole group of voxels that share them), [15] zero. */
@@ -138,8 +139,8 @@ typedef struct bs_m2v_params {
   int32_t wn_tree;     /* 0: the reference's own tree — the top-down SAH build of AABBTree::top_down::<Area>
                           with 3 triangles per leaf (aabb_tree.rs:118-199, 422-514, 636-644), one traversal
                           per voxel summing wn(left) + wn(right) as fast_wn recurses (aabb_tree.rs:662-691):
-                          signs equal the reference's bit for bit.  1: this library's PLOC tree with a
-                          warp-coherent traversal (faster; signs differ only where the winding number is
+                          signs equal the reference's bit for bit.  1: this library's PLOC tree, one cut
+                          of it for 32 voxels (faster; signs differ only where the winding number is
                           within the far-field approximation error of the threshold).  All meshes of a
                           batch use the same value. */
 } bs_m2v_params;
