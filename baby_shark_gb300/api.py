@@ -126,6 +126,7 @@ class Context:
         out["wn_tree"] = "reference" if a[12] == 0 else "fast"
         out["wn_far_warp_sections"] = a[13]
         out["wn_exact_warp_sections"] = a[14]
+        out["wn_left_to_traversal"] = a[15]
         return out
 
 

@@ -65,6 +65,7 @@ struct M2VStats {
   unsigned long long wn_visits;      // warp-level node visits of the winding-number pass
   unsigned long long wn_far;         // warp-level far-field evaluations (internal + leaf dipoles)
   unsigned long long wn_exact;       // warp-level exact solid angles
+  unsigned long long wn_left;        // warps that the filter left to the traversal
   unsigned long long n_eval;         // (voxel, sub-triangle) pairs left after culling
   unsigned long long area16;         // surface in sixteenths of a squared voxel and
   unsigned long long n_uncullable;   // about how many sub-triangles are never culled (for choosing the distance pass)
@@ -1584,6 +1585,7 @@ __global__ void __launch_bounds__(WN_THREADS, REST_BLOCKS) k_wn_sign_rest(const 
   auto walk = [&](int mesh, uint64_t i0, bool count) {
     const uint64_t i = i0 + lane, a1 = act_base[mesh + 1];
     const MeshInfo M = mi[mesh];
+    if (lane == 0) atomicAdd(&stats[mesh].wn_left, 1ull);
     wn_warp<2>(act, i, i < a1, a1 - 1, origins, values, inodes + 5 * uint64_t(inode_base[mesh]),
                leaves + 5 * uint64_t(tri_base[mesh]), nullptr, nullptr, int(M.n_tri), M.h, M.beta, M.thresh,
                stats + mesh, stk, count);
@@ -2268,14 +2270,14 @@ static std::vector<bs_volume*> batch_core(bs_ctx* ctx, const float* d_xyz, const
   // join the tree build; the triangles are freed after it
   BS_CUDA(cudaStreamWaitEvent(s, built.e, 0));
   T.reset();
-  unsigned long long rt_cnt[6] = {0, 0, 0, 0, 0, 0};
+  unsigned long long rt_cnt[RT_COUNTERS] = {};
   if (na > 0 && ref_tree) {
     std::vector<RefSignMesh> rm(K);
     for (int m = 0; m < K; ++m) rm[m] = RefSignMesh{rt.h_roots[m], mi[m].h, mi[m].beta, mi[m].thresh};
     DBuf<RefSignMesh> d_rm(ctx, K);
-    DBuf<unsigned long long> d_cnt(ctx, 6);
+    DBuf<unsigned long long> d_cnt(ctx, RT_COUNTERS);
     BS_CUDA(cudaMemcpyAsync(d_rm.p, rm.data(), K * sizeof(RefSignMesh), cudaMemcpyHostToDevice, s));
-    BS_CUDA(cudaMemsetAsync(d_cnt.p, 0, 6 * sizeof(unsigned long long), s));
+    BS_CUDA(cudaMemsetAsync(d_cnt.p, 0, sizeof rt_cnt, s));
     ref_tree_sign(ctx, rt, act.p, voff.p, nb, na, act_base.p, leaf_base.p, K, d_rm.p, origins.p, values.p, d_cnt.p);
     read_back(ctx, rt_cnt, d_cnt.p, sizeof rt_cnt);
     if (rt_cnt[3]) fail(BS_ERR_CAPACITY, "winding-number traversal stack overflow");
@@ -2319,7 +2321,7 @@ static std::vector<bs_volume*> batch_core(bs_ctx* ctx, const float* d_xyz, const
 #undef BS_WN3
   }
   read_back(ctx, hst.data(), st.p, K * sizeof(M2VStats));
-  uint64_t n_vp = 0, n_p = 0, visits = 0, far = 0, exact = 0, n_ev = 0;
+  uint64_t n_vp = 0, n_p = 0, visits = 0, far = 0, exact = 0, left = 0, n_ev = 0;
   for (int m = 0; m < K; ++m) {
     if (hst[m].error == 3) fail(BS_ERR_CAPACITY, "winding-number traversal stack overflow");
     n_vp += hst[m].n_vpairs;
@@ -2328,11 +2330,13 @@ static std::vector<bs_volume*> batch_core(bs_ctx* ctx, const float* d_xyz, const
     visits += hst[m].wn_visits;
     far += hst[m].wn_far;
     exact += hst[m].wn_exact;
+    left += hst[m].wn_left;
   }
   if (ref_tree) {  // per voxel rather than per warp
     visits = rt_cnt[0];
     far = rt_cnt[1];
     exact = rt_cnt[2];
+    left = rt_cnt[6];
   }
   ctx->last_stats[0] = nt;
   ctx->last_stats[1] = ns;
@@ -2349,6 +2353,7 @@ static std::vector<bs_volume*> batch_core(bs_ctx* ctx, const float* d_xyz, const
   ctx->last_stats[12] = ref_tree ? 0 : 1;
   ctx->last_stats[13] = ref_tree ? rt_cnt[4] : 0;
   ctx->last_stats[14] = ref_tree ? rt_cnt[5] : 0;
+  ctx->last_stats[15] = left;
 
   // hand out the volumes
   std::vector<bs_volume*> vols(K, nullptr);

@@ -1142,6 +1142,7 @@ __global__ void __launch_bounds__(32 * SIGN_WARPS) k_rt_sign_exact(const uint32_
     const bool ok = mine != NO_VOXEL;
     const unsigned valid = __ballot_sync(FULL, ok);
     if (!valid) continue;  // the end of a block
+    if (lane == 0) atomicAdd(counters + 6, (unsigned long long)__popc(valid));
     const RefSignMesh M = meshes[m];
     const uint32_t other = __shfl_sync(FULL, mine, __ffs(valid) - 1), v = ok ? mine : other;
     const uint32_t b = v >> 9, o = v & 511;

@@ -56,10 +56,12 @@ struct RefSignMesh {
 // [leaf_base[m], leaf_base[m+1]) and act[act_base[m], act_base[m+1])) with the
 // winding number of their grid points: values[v] = +|d| when wn < thresh,
 // else -|d| (mesh_to_volume.rs:245-280).  sign_filter.cu settles all but a few
-// voxels; the rest take the exact traversal.  counters (device, 6 x u64,
-// accumulated): node visits, far-field evaluations and exact solid angles of
-// the voxels' own cuts, stack overflows, far-field evaluations and solid
-// angles as the kernel runs them (one for a whole group of voxels).
+// voxels; the rest take the exact traversal.  counters (device,
+// RT_COUNTERS x u64, accumulated): node visits, far-field evaluations and exact
+// solid angles of the voxels' own cuts, stack overflows, far-field evaluations
+// and solid angles as the kernel runs them (one for a whole group of voxels),
+// voxels left to the exact traversal.
+constexpr int RT_COUNTERS = 7;
 void ref_tree_sign(bs_ctx* ctx, const RefTrees& t, const uint32_t* act, const uint32_t* voff, uint64_t n_bricks,
                    uint64_t n_act, const uint32_t* d_act_base, const uint32_t* d_leaf_base, int K,
                    const RefSignMesh* d_meshes, const int4* origins, float* values, unsigned long long* d_counters);

@@ -94,7 +94,9 @@ bs_status bs_ctx_last_stats(const bs_ctx* ctx, uint64_t* out8);
  * whichever kernel walks it), [12] which tree
  * (0 the reference's, 1 PLOC), [13] and [14] on the reference's tree the
  * far-field evaluations and solid angles as the pass runs them (once for a
- * whole group of voxels that share them), [15] zero. */
+ * whole group of voxels that share them), [15] what a mesh -> volume call's sign
+ * filter left to the traversal: voxels on the reference's tree, warps of 32 on
+ * the PLOC tree (0 with the order-3 expansion, which has no filter). */
 enum bs_stats_kind {
   BS_STATS_NONE = 0,
   BS_STATS_MESH_TO_VOLUME = 1,

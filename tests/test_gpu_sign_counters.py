@@ -13,7 +13,7 @@ from tests.gpu_common import context, unpack_mask
 from tests.test_gpu_fast_sign import MORTON
 from tests.test_gpu_fast_sign import convert as convert_fast
 from tests.test_gpu_sign_filter import convert as convert_reference
-from tests.test_gpu_sign_filter import shapes
+from tests.test_gpu_sign_filter import shapes, soup
 
 pytestmark = pytest.mark.gpu
 KEYS = {"fast": ("wn_warp_visits", "wn_far", "wn_exact"), "reference": ("wn_far", "wn_exact")}
@@ -24,6 +24,9 @@ def cases():
     out = {k: (*s[k], 2.0, 0.2) for k in ("torus", "on_grid", "degenerate", "tiny", "out_of_range", "coarse", "few2")}
     # every node near: the pending nodes of 32 voxels outgrow the filter's stacks
     out["all_near"] = (*synthetic.torus(1.0, 0.3, 400, 200, 0.02, seed=3), 0.2, 1, 500.0, 0.2)
+    # random triangles: values on either side of the threshold and close to it
+    rng = np.random.default_rng(0)
+    out["heap"] = (*soup(rng.normal(size=(20000, 1, 3)) * 0.3 + rng.normal(size=(20000, 3, 3)) * 0.02), 0.03, 2, 2.0, 0.2)
     # a threshold at the outside's value: half of the groups cannot be settled,
     # and after the first ones the filter gives the mesh up
     out["outside_value"] = (*synthetic.torus(1.0, 0.3, 256, 128, 0.02, seed=3), 0.006, 3, 2.0, 0.0)
