@@ -6,9 +6,10 @@
 // needs only the side of the threshold its sum lies on
 // (mesh_to_volume.rs:264-271).  This pass walks the same cut and evaluates it
 // in cheaper arithmetic with a bound on how far the traversal's float32 sum
-// can be (sign_filter.cuh); the warps whose voxels' sides it cannot settle, or
-// whose cut it has no room for, are listed and traversed (k_wn_sign_rest), so the signs are
-// the traversal's.
+// can be (sign_filter.cuh).  The warps whose voxels' sides it cannot settle, or
+// whose cut it has no room for, are listed and traversed (k_wn_sign_rest), as
+// are those of a mesh out of its range or that it gives up, so the signs are the
+// traversal's.
 //
 // What makes it cheap: nodes are tested 32 at a time, one per lane, against
 // the bounding sphere and box of the voxels (of up to 256 consecutive ones

@@ -23,10 +23,11 @@
 // denominator, as fractions of |a||b||c|, differ by less than 256 u from the
 // reference's, which moves the angle by at most 1.5 * 256 u / max(|num|,
 // |den|); with the arctangent's 1e-5 that is below 1.4e-4 / max(..) for twice
-// the angle.  A voxel is left undecided where that argument ends: near the
-// branch cut (den < 0, |num| small), at a vertex or edge, outside the range
-// of distances where no float32 product of either formula over- or
-// underflows, or where any value is NaN.
+// the angle.  Where that argument ends, near the branch cut (den < 0, |num|
+// small) and at a vertex or edge, the callers take the exact formula or a wider
+// bound.  A voxel is left undecided outside the range of distances where no
+// float32 product of either formula over- or underflows, or where any value is
+// NaN.
 #pragma once
 
 #include "bs_internal.cuh"
