@@ -196,20 +196,21 @@ __device__ __forceinline__ int ranked(const uint2* __restrict__ m, int o) {
   return (e.x & bit) ? int(e.y + __popc(e.x & (bit - 1u))) : -1;
 }
 
-// Crossing points and normals (dual_contouring.rs:249-313): one warp per
+// Crossing points and normals (dual_contouring.rs:249-313): `split` warps per
 // leaf, its crossings (directions, then voxels in ascending order) listed and
 // taken 32 at a time, so points are written in order.
 template <bool TILES>
 __global__ void __launch_bounds__(32 * DC_WARPS) k_dc_edge_points(DcVol V, uint64_t n, const uint2* __restrict__ em,
                                                                   const uint32_t* __restrict__ coff,
-                                                                  float* __restrict__ pts, DcStats* st) {
+                                                                  float* __restrict__ pts, DcStats* st,
+                                                                  uint32_t split) {
   __shared__ uint16_t list[DC_WARPS][3 * 512];
   __shared__ int nbs[DC_WARPS][27];
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
-  const uint64_t l = blockIdx.x * uint64_t(DC_WARPS) + wi;
+  const uint64_t gw = blockIdx.x * uint64_t(DC_WARPS) + wi, l = gw / split;
   if (l >= n) return;
-  const uint32_t c0 = coff[l * 3], cnt = coff[l * 3 + 3] - c0;
-  if (cnt == 0) return;
+  const uint32_t c0 = coff[l * 3], cnt = coff[l * 3 + 3] - c0, first = 32 * uint32_t(gw % split);
+  if (cnt <= first) return;
   if (lane < 27) nbs[wi][lane] = V.nbr[l * 27 + lane];
   for (int k = lane; k < 48; k += 32) {
     const uint2 e = em[l * 48 + k];
@@ -219,7 +220,7 @@ __global__ void __launch_bounds__(32 * DC_WARPS) k_dc_edge_points(DcVol V, uint6
   __syncwarp();
   const int* nb = nbs[wi];
   const int4 org = V.org[l];
-  for (uint32_t i = lane; i < cnt; i += 32) {
+  for (uint32_t i = first + lane; i < cnt; i += 32 * split) {
     const int code = list[wi][i], dir = code >> 9, o = code & 511;
     const int x = o >> 6, y = (o >> 3) & 7, z = o & 7;
     const int x2 = x + (dir == 0), y2 = y + (dir == 1), z2 = z + (dir == 2);
@@ -286,29 +287,28 @@ __device__ __forceinline__ uint32_t list_cells(const uint2* __restrict__ cellm, 
 }
 
 // The particle solver (dual_contouring.rs:429-458), a lane per cell and
-// CELL_SPLIT warps per leaf.  Its 50 dependent iterations set the time, so
+// `split` warps per leaf.  Its 50 dependent iterations set the time, so
 // the quotients by the number of crossings share one reciprocal and a leaf's
-// cells are spread over two warps.  (Crossings copied to shared memory instead
+// cells are spread over two warps or more.  (Crossings copied to shared memory instead
 // of read through L1: 0.40 against 0.14 ms on 57 k leaves, the 9 KB per warp
 // leave too few warps resident.)
-constexpr int CELL_SPLIT = 2;
 __global__ void __launch_bounds__(32 * DC_WARPS) k_dc_cell_points(DcVol V, uint64_t n, const uint2* __restrict__ em,
                                                                   const uint32_t* __restrict__ coff,
                                                                   const float* __restrict__ pts,
                                                                   const uint2* __restrict__ cellm,
                                                                   const uint32_t* __restrict__ celloff,
-                                                                  float* __restrict__ cells) {
+                                                                  float* __restrict__ cells, uint32_t split) {
   __shared__ uint16_t list[DC_WARPS][512];
   __shared__ int nbs[DC_WARPS][27];
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
-  const uint64_t gw = blockIdx.x * uint64_t(DC_WARPS) + wi, l = gw / CELL_SPLIT;
+  const uint64_t gw = blockIdx.x * uint64_t(DC_WARPS) + wi, l = gw / split;
   if (l >= n) return;
-  const uint32_t cnt = list_cells(cellm, l, list[wi]), first = 32 * uint32_t(gw % CELL_SPLIT);
+  const uint32_t cnt = list_cells(cellm, l, list[wi]), first = 32 * uint32_t(gw % split);
   if (cnt <= first) return;
   if (lane < 27) nbs[wi][lane] = V.nbr[l * 27 + lane];
   __syncwarp();
   const int* nb = nbs[wi];
-  for (uint32_t ci = first + lane; ci < cnt; ci += 32 * CELL_SPLIT) {
+  for (uint32_t ci = first + lane; ci < cnt; ci += 32 * split) {
     const int o = list[wi][ci];
     const int x = o >> 6, y = (o >> 3) & 7, z = o & 7;
     const float2* ip[12];
@@ -402,18 +402,18 @@ __global__ void __launch_bounds__(32 * DC_WARPS) k_dc_cell_qef(DcVol V, uint64_t
                                                                const float* __restrict__ pts,
                                                                const uint2* __restrict__ cellm,
                                                                const uint32_t* __restrict__ celloff,
-                                                               float* __restrict__ cells) {
+                                                               float* __restrict__ cells, uint32_t split) {
   __shared__ uint16_t list[DC_WARPS][512];
   __shared__ int nbs[DC_WARPS][27];
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
-  const uint64_t l = blockIdx.x * uint64_t(DC_WARPS) + wi;
+  const uint64_t gw = blockIdx.x * uint64_t(DC_WARPS) + wi, l = gw / split;
   if (l >= n) return;
-  const uint32_t cnt = list_cells(cellm, l, list[wi]);
-  if (cnt == 0) return;
+  const uint32_t cnt = list_cells(cellm, l, list[wi]), first = 32 * uint32_t(gw % split);
+  if (cnt <= first) return;
   if (lane < 27) nbs[wi][lane] = V.nbr[l * 27 + lane];
   __syncwarp();
   const int* nb = nbs[wi];
-  for (uint32_t ci = lane; ci < cnt; ci += 32) {
+  for (uint32_t ci = first + lane; ci < cnt; ci += 32 * split) {
     const int o = list[wi][ci];
     const int x = o >> 6, y = (o >> 3) & 7, z = o & 7;
     double mp[3] = {0.0, 0.0, 0.0}, ata[3][3] = {{0.0}}, atb[3] = {0.0, 0.0, 0.0};
@@ -560,6 +560,22 @@ __global__ void __launch_bounds__(32 * DC_WARPS) k_dc_quads(DcVol V, uint64_t n,
 // Launches shared with dc_noalloc.cu (tiles: the volume has active tiles).
 static inline unsigned dc_blocks(uint64_t n) { return unsigned((n + DC_WARPS - 1) / DC_WARPS); }
 
+// Warps per leaf of the passes that compute values: `least` where the leaves
+// fill the SMs, doubled up to 16 (all 512 cells of a leaf at once) while there
+// are 64 warps or fewer to an SM, since a warp goes through a crowded leaf's
+// cells 32 at a time.  With one warp (two for the particles) throughout
+// against this, cell pass in ms, QEF / particles: 64 crowded leaves 0.774 /
+// 0.304 against 0.071 / 0.055; 1,440 of a surface 0.301 / 0.096 against 0.200 /
+// 0.069; 5,858 (above the line) 0.66 / 0.10 on both sides.
+static uint32_t dc_split(uint64_t n, uint32_t least) {
+  int device = 0, n_sm = 0;
+  BS_CUDA(cudaGetDevice(&device));
+  BS_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, device));
+  uint32_t split = least;
+  while (split < 16 && n * split * 2 <= uint64_t(n_sm) * 64) split *= 2;
+  return split;
+}
+
 void launch_dc_prepare(const DcVol& V, LeafHash hash, uint64_t n, int* nbr, uint32_t* sgn, cudaStream_t s) {
   k_dc_neighbours<<<unsigned((27 * n + 255) / 256), 256, 0, s>>>(V.org, hash, n, nbr);
   k_dc_signs<<<dc_blocks(n), 32 * DC_WARPS, 0, s>>>(V.val, n, sgn);
@@ -573,18 +589,20 @@ void launch_dc_masks(bool tiles, const DcVol& V, uint64_t n, uint2* em, uint32_t
 }
 void launch_dc_edge_points(bool tiles, const DcVol& V, uint64_t n, const uint2* em, const uint32_t* coff, float* pts,
                            DcStats* st, cudaStream_t s) {
+  const uint32_t split = dc_split(n, 1);
   if (tiles)
-    k_dc_edge_points<true><<<dc_blocks(n), 32 * DC_WARPS, 0, s>>>(V, n, em, coff, pts, st);
+    k_dc_edge_points<true><<<dc_blocks(n * split), 32 * DC_WARPS, 0, s>>>(V, n, em, coff, pts, st, split);
   else
-    k_dc_edge_points<false><<<dc_blocks(n), 32 * DC_WARPS, 0, s>>>(V, n, em, coff, pts, st);
+    k_dc_edge_points<false><<<dc_blocks(n * split), 32 * DC_WARPS, 0, s>>>(V, n, em, coff, pts, st, split);
 }
 void launch_dc_cell_points(int mode, const DcVol& V, uint64_t n, const uint2* em, const uint32_t* coff,
                            const float* pts, const uint2* cellm, const uint32_t* celloff, float* cells,
                            cudaStream_t s) {
+  const uint32_t split = dc_split(n, mode == 1 ? 1 : 2);
   if (mode == 1)
-    k_dc_cell_qef<<<dc_blocks(n), 32 * DC_WARPS, 0, s>>>(V, n, em, coff, pts, cellm, celloff, cells);
+    k_dc_cell_qef<<<dc_blocks(n * split), 32 * DC_WARPS, 0, s>>>(V, n, em, coff, pts, cellm, celloff, cells, split);
   else
-    k_dc_cell_points<<<dc_blocks(n * CELL_SPLIT), 32 * DC_WARPS, 0, s>>>(V, n, em, coff, pts, cellm, celloff, cells);
+    k_dc_cell_points<<<dc_blocks(n * split), 32 * DC_WARPS, 0, s>>>(V, n, em, coff, pts, cellm, celloff, cells, split);
 }
 void launch_dc_quads(const DcVol& V, uint64_t n, const uint2* em, const uint32_t* coff, const uint2* cellm,
                      const uint32_t* celloff, const float* cells, float h, uint64_t* vcount, const uint64_t* voff,
