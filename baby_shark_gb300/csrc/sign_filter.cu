@@ -517,12 +517,16 @@ void ref_tree_sign(bs_ctx* ctx, const RefTrees& t, const uint32_t* act, const ui
                                   t.rad_l.p, t.tri.p, d_act_base, und.p, n_und.p, d_counters)))
   int n_sm = 0;
   BS_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, ctx->device));
-  // A brick's warps take its groups in turn, so where the bricks are too few
-  // for the SMs' warps (24 each) they get more of them, up to one per group: 124
-  // bricks with 4, 8, 16 warps 8.7, 5.0, 3.5 ms (accuracy scale 8); 947 bricks
-  // with 4, 8 warps 0.70, 0.73 ms.
+  // A brick's warps take its groups in turn, and the busiest brick's turns set
+  // the time, so where the bricks are few they get more warps, up to one per
+  // group, while there are 64 warps or fewer to an SM.  With 4 / 8 / 16 warps:
+  // 124 bricks of a torus (accuracy scale 8) 8.7 / 5.0 / 3.5 ms; 543 of random
+  // triangles 9.7 / 5.8 / 3.6; 512 of small boxes 1.65 / 1.05 / -; 545 of a torus
+  // 0.415 / 0.346 / 0.395; 960 of a torus 0.409 / 0.426 / -; 1,451 (past the
+  // line) 0.436 / 0.524 / -.  (24 warps fit an SM at a time; a line there: a
+  // batch of eight meshes, two of them crowded, 648 bricks, 2.32 against 1.31 ms.)
   int warps_of = ctx->tune_wn_warps;
-  while (warps_of < 16 && n_bricks * 2 * warps_of <= uint64_t(n_sm) * 24) warps_of *= 2;
+  while (warps_of < 16 && n_bricks * 2 * warps_of <= uint64_t(n_sm) * 64) warps_of *= 2;
   if (warps_of == 2)
     BS_RT_SIGN(2);
   else if (warps_of == 8)

@@ -75,3 +75,19 @@ def test_few_bricks_get_more_warps():
         _, times[warps] = stages(lambda: convert_reference(v, f, 0.05, 1, 4.0, 0.2), ("k_rt_sign",))
     print("k_rt_sign %.3f ms with 4 warps, %.3f ms with 8" % (times[4], times[8]))
     assert 0 < times[4] <= 1.2 * times[8]
+
+
+def test_some_hundred_crowded_bricks_get_more_warps():
+    """As above for five hundred bricks among random triangles, where a group
+    of voxels takes long and the busiest brick sets the time."""
+    rng = np.random.default_rng(3)
+    t = rng.normal(size=(100000, 1, 3)) * 0.3 + rng.normal(size=(100000, 3, 3)) * 0.01
+    v, f = t.reshape(-1, 3).astype(np.float32), np.arange(300000, dtype=np.uint32).reshape(-1, 3)
+    times = {}
+    for warps in (8, 4):  # four is a context's own
+        context().set_launch_shape(0, warps, 0)
+        vol, times[warps] = stages(lambda: convert_reference(v, f, 0.037, 1, 2.0, 0.2), ("k_rt_sign",))
+    n = vol.counts()["leaves"]
+    print("%d bricks: k_rt_sign %.3f ms with 4 warps, %.3f ms with 8" % (n, times[4], times[8]))
+    assert 456 < n < 608  # from 24 warps to an SM with 8 warps a brick to 64 with 16
+    assert 0 < times[4] <= 1.2 * times[8]
