@@ -2091,12 +2091,16 @@ static std::vector<bs_volume*> batch_core(bs_ctx* ctx, const float* d_xyz, const
   ctx->dist_on_patches = patches;
   DBuf<Patch> pat;
   uint64_t n_list = ns;  // entries of the lists' kind: sub-triangles or patches
+  uint32_t pat_split = 1;  // threads per patch of the passes that fill the lists
   if (patches) {
     poff = DBuf<uint32_t>(ctx, nt + 1);
     exclusive_scan(ctx, npat.p, poff.p, nt + 1);
     uint32_t total_p = 0;
     read_back(ctx, &total_p, poff.p + nt, sizeof(uint32_t));
     n_list = total_p;
+    int n_sm = 0;
+    BS_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, ctx->device));
+    while (pat_split < 32 && n_list * pat_split * 2 <= uint64_t(n_sm) * 512) pat_split *= 2;
     pat = DBuf<Patch>(ctx, n_list);
     BS_KERNEL(ctx, "k_patches", (k_patches<<<blocks(n_list, 128), 128, 0, s>>>(T.p, nsub.p, soff.p, poff.p, nt, n_list, d_mi.p, S.p, pat.p, st.p)));
     poff.reset();
@@ -2109,7 +2113,7 @@ static std::vector<bs_volume*> batch_core(bs_ctx* ctx, const float* d_xyz, const
   DBuf<uint32_t> cnt(ctx, DC + 1), pair_off(ctx, DC + 1), flag(ctx, D + 1), bidx(ctx, D + 1);
   BS_CUDA(cudaMemsetAsync(cnt.p, 0, (DC + 1) * sizeof(uint32_t), s));
   if (patches)
-    BS_KERNEL(ctx, "k_count_patches", (k_count_patches<<<blocks(n_list, 256), 256, 0, s>>>(pat.p, n_list, S.p, d_dirs.p, d_db.p, cnt.p, st.p)));
+    BS_KERNEL(ctx, "k_count_patches", ((pat_split > 1 ? k_count_patches<true> : k_count_patches<false>)<<<blocks(n_list * pat_split, 256), 256, 0, s>>>(pat.p, n_list, S.p, d_dirs.p, d_db.p, cnt.p, st.p, pat_split)));
   else
     BS_KERNEL(ctx, "k_count_pairs", (k_count_pairs<<<blocks(ns, 256), 256, 0, s>>>(S.p, ns, d_dirs.p, d_db.p, cnt.p, st.p)));
   exclusive_scan(ctx, cnt.p, pair_off.p, DC + 1);
@@ -2148,7 +2152,7 @@ static std::vector<bs_volume*> batch_core(bs_ctx* ctx, const float* d_xyz, const
     pair_off.reset();
     bidx.reset();
     if (patches)
-      BS_KERNEL(ctx, "k_fill_patches", (k_fill_patches<<<blocks(n_list, 256), 256, 0, s>>>(pat.p, n_list, S.p, d_dirs.p, d_db.p, cnt.p, list.p)));
+      BS_KERNEL(ctx, "k_fill_patches", ((pat_split > 1 ? k_fill_patches<true> : k_fill_patches<false>)<<<blocks(n_list * pat_split, 256), 256, 0, s>>>(pat.p, n_list, S.p, d_dirs.p, d_db.p, cnt.p, list.p, pat_split)));
     else
       BS_KERNEL(ctx, "k_fill_pairs", (k_fill_pairs<<<blocks(ns, 256), 256, 0, s>>>(S.p, ns, d_dirs.p, d_db.p, cnt.p, list.p)));
     cnt.reset();

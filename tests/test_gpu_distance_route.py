@@ -89,3 +89,40 @@ def test_every_launch_shape_of_both_passes_matches_oracle(band, patches):
         rep = compare_volumes(vol.export(), o, check_inactive=True)
         assert rep["leaf_set_equal"] and rep["mask_mismatch_leaves"] == rep["value_mismatch"] == 0, rep
         assert rep["sign_mismatch"] == rep["inactive_mismatch"] == 0 and rep["active"] > 0, rep
+
+
+def of_every_split():
+    """Meshes whose patches' lists are filled by 32, 16, ... 1 threads per patch, with voxel size and band."""
+    return {"80": (synthetic.icosphere(1, 1.0, 0.0, seed=1), 0.1625, 5),
+            "1280": (synthetic.icosphere(3, 1.0, 0.0, seed=1), 0.03, 4),
+            "5120": (synthetic.icosphere(4, 1.0, 0.005, seed=1), 0.015, 4),
+            "9216": (synthetic.torus(1.0, 0.3, 96, 48, 0.02, seed=5), 0.02, 4),
+            "65536": (synthetic.torus(1.0, 0.3, 256, 128, 0.02, seed=5), 0.0075, 4)}
+
+
+@pytest.mark.parametrize("name", ["80", "1280", "5120", "9216", "65536"])
+def test_lists_of_patches_are_complete_at_every_split(name):
+    mesh, h, band = of_every_split()[name]
+    vol, took = convert(mesh, h, band)
+    assert took
+    assert_same(vol, mesh, h, band)
+
+
+def test_lists_of_few_large_patches_cost_less_than_the_pass():
+    """80 triangles, dozens of bricks each: filling the lists must leave most of
+    the time to the distances."""
+    mesh, h, band = of_every_split()["80"]
+    ctx = context()
+    best = {}
+    ctx.set_stage_timing(True)
+    try:
+        for _ in range(6):
+            ctx.stage_times(reset=True)
+            bs.MeshToVolume(ctx).with_voxel_size(h).with_narrow_band_width(band).convert(mesh)
+            for k, (ms, _) in ctx.stage_times(reset=True).items():
+                best[k] = min(best.get(k, 1e9), ms)
+    finally:
+        ctx.set_stage_timing(False)
+    lists = best["k_count_patches"] + best["k_fill_patches"]
+    print("lists %.3f ms, distances %.3f ms" % (lists, best["k_patch_distance"]))
+    assert lists <= 0.75 * best["k_patch_distance"]
