@@ -547,6 +547,8 @@ bs_corner_table* corner_table_from_device_soup(bs_ctx* ctx, const float* d_pts, 
     BS_KERNEL(ctx, "k_fans", (k_fans<<<nbc(nv + 1, 128), 128, 0, s>>>(vcorner.p, deleted.p, vstart.p, vlist.p, copp.p, nv, fan.p,
                                                                    cval.p, extra.p)));
     scan_ex(ctx, extra.p, extra_off.p, nv + 1);
+    resize_for_copy(t->cvertex, nc);  // while the kernels run
+    resize_for_copy(t->copp, nc);
     read_back(ctx, &n_extra, extra_off.p + nv, sizeof n_extra);
     if (n_extra)
       BS_KERNEL(ctx, "k_split", (k_split<<<nbc(nv, 128), 128, 0, s>>>(deleted.p, vstart.p, vlist.p, fan.p, cval.p, extra_off.p, nv, pos.p,
@@ -556,8 +558,6 @@ bs_corner_table* corner_table_from_device_soup(bs_ctx* ctx, const float* d_pts, 
   resize_for_copy(t->pos, slots * 3);
   resize_for_copy(t->deleted, slots);
   resize_for_copy(t->vcorner, slots);
-  resize_for_copy(t->cvertex, nc);
-  resize_for_copy(t->copp, nc);
   if (slots) {
     BS_CUDA(cudaMemcpyAsync(t->pos.data(), pos.p, slots * 3 * sizeof(float), cudaMemcpyDeviceToHost, s));
     BS_CUDA(cudaMemcpyAsync(t->deleted.data(), deleted.p, slots, cudaMemcpyDeviceToHost, s));
